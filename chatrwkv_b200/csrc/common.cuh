@@ -21,8 +21,8 @@ static inline int rwkv_launch_status() {
 // in the stream drains; kernels order themselves with griddepcontrol.wait.  RWKV_B200_PDL=0
 // in the environment turns the attribute off.
 template <typename... KArgs, typename... Args>
-static inline int rwkv_launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                                  Args... args) {
+static inline int rwkv_launch_pdl_clustered(unsigned cluster, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                            const Args&... args) {
     static int use_pdl = -1;
     if (use_pdl < 0) {
         const char* e = getenv("RWKV_B200_PDL");
@@ -33,14 +33,28 @@ static inline int rwkv_launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 bloc
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (use_pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {                      // along x
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = cluster;
+        attr[n].val.clusterDim.y = 1;
+        attr[n++].val.clusterDim.z = 1;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = use_pdl ? 1 : 0;
+    cfg.numAttrs = n;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
     if (e != cudaSuccess) { cudaGetLastError(); return RWKV_ERR_LAUNCH; }
     return RWKV_OK;
+}
+template <typename... KArgs, typename... Args>
+static inline int rwkv_launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                  const Args&... args) {
+    return rwkv_launch_pdl_clustered(1, kernel, grid, block, smem, st, args...);
 }
 
 static inline int rwkv_sm_count() {       // of the current device

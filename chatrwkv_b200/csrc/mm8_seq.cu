@@ -5,9 +5,12 @@
 // with x' = x*ry, SX = sum_j x, SXR = sum_j x', SXMY = sum_j x*my (per row i).
 //
 // This file holds the shape-agnostic CUDA-core kernel (any B, N, M, any stride or
-// alignment).  It is the path for ragged or misaligned operands and for small B.
+// alignment; the path for misaligned operands, fp32 and one row) and the choice between it and
+// the tensor-core kernels (mm8_seq_i8.cu, mm8_seq_tc.cu).
 #include "common.cuh"
+#include "mm8_seq_i8.h"
 #include "seq_epi.cuh"
+#include <algorithm>
 
 namespace {
 
@@ -103,20 +106,23 @@ int rwkv_mm8_seq_tc(int64_t B, int64_t N, int64_t M, const void* x, int64_t x_st
 
 extern "C" void rwkv_mm8_seq_tc_set_single(int single);
 void rwkv_mm8_seq_tc_set_no_pair(int no_pair);
+static int g_seq_single = 0;
 static int g_seq_path = 0;      // 0 = automatic, 1 = CUDA cores only, 2 = tensor cores whenever the layout allows
-// bit 2 (value 4) of `path`: the tensor-core kernel multiplies fp16(x*ry) in one pass instead of the exact
-// hi + lo pair; bit 3 (value 8): one CTA per output tile always (never the CTA-pair form; same results)
+// bit 2 (value 4) of `path`: one pass of the fp16 tensor-core kernel with fp16(x*ry); bit 3 (value 8): one CTA per output tile always (never the CTA-pair form; same results)
 extern "C" void rwkv_mm8_seq_set_path(int path) {
     g_seq_path = path & 3;
-    rwkv_mm8_seq_tc_set_single((path & 4) != 0);
+    g_seq_single = (path & 4) != 0;
+    rwkv_mm8_seq_tc_set_single(g_seq_single);
     rwkv_mm8_seq_tc_set_no_pair((path & 8) != 0);
+    rwkv_mm8_seq_i8_set_form((path & 8) != 0 ? 1 : 0);
 }
-constexpr int kTcMinRows = 8;   // below this the CUDA-core kernel; from here on the 128-row tensor-core tile (mostly padding up to
-                                // 64 rows, but 4x faster than the CUDA-core kernel already at 16 rows: W is converted once per CTA)
+constexpr int kI8MinRows = 2;   // one row is mm8_one's work; from two on the integer tensor-core kernel (4096 x 4096: 11 us)
+constexpr int kTcMinRows = 8;   // rows that TMA cannot fetch: below this the CUDA-core kernel, from here on the 128-row fp16 tile
+                                // (4x faster than the CUDA-core kernel already at 16 rows: W is converted once per CTA)
 
 extern "C" size_t rwkv_mm8_seq_workspace_bytes(int64_t B, int64_t N, int64_t M) {
     if (B < 1 || N < 1 || M < 1) return 0;
-    return rwkv_mm8_seq_tc_workspace_bytes(B, N, M);
+    return std::max(rwkv_mm8_seq_tc_workspace_bytes(B, N, M), rwkv_mm8_seq_i8_workspace_bytes(1, B, N, &M));
 }
 
 extern "C" int rwkv_mm8_seq_epi(int64_t B, int64_t N, int64_t M, const void* x, int64_t x_stride,
@@ -133,6 +139,11 @@ extern "C" int rwkv_mm8_seq_epi(int64_t B, int64_t N, int64_t M, const void* x, 
     epi.mode = epilogue; epi.out_scale = out_scale; epi.aux = aux; epi.aux_stride = aux_stride; epi.aux2 = aux2; epi.aux2_stride = aux2_stride;
     const int erc = seq_epi_check(epi);
     if (erc != RWKV_OK) return erc;
+    if (g_seq_path != 1 && !g_seq_single && workspace != nullptr && dtype == RWKV_F16 && (B >= kI8MinRows || g_seq_path == 2)) {
+        const SeqI8Problem p = {x, x_stride, w, w_stride, mx, rx, my, ry, y, y_stride, M, epi};
+        const int rc = rwkv_mm8_seq_i8(1, &p, B, N, workspace, workspace_bytes, stream);
+        if (rc != RWKV_ERR_UNSUPPORTED && rc != RWKV_ERR_WORKSPACE) return rc;   // else: the general kernels below
+    }
     if (g_seq_path != 1 && workspace != nullptr && (B >= kTcMinRows || g_seq_path == 2)) {
         const int rc = rwkv_mm8_seq_tc(B, N, M, x, x_stride, w, w_stride, mx, rx, my, ry, dtype, y, y_stride, epi,
                                        workspace, workspace_bytes, stream);

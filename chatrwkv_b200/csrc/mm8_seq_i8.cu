@@ -1,0 +1,793 @@
+// mm8_seq on the integer path of the 5th-generation tensor cores (tcgen05 kind::i8): the packed matrix is multiplied as
+// the bytes it is stored as.
+//
+//   y[t,n] = rx[n] * sum_k x'[t,k] (w[k,n] - 128) + rx[n]*128.5*SXR[t] + mx[n]*SX[t] + SXMY[t]
+//
+// with x' = x*ry, SX = sum_k x, SXR = sum_k x', SXMY = sum_k x*my (per row t), the factorisation of mm8_one.
+//   * x' becomes a 24-bit fixed-point integer per row (the scale is the power of two that takes the row's largest
+//     magnitude into [2^22, 2^23), so the fp32 products are scaled exactly and rounded once, to 2^-23 .. 2^-22 of the
+//     row's maximum) and enters as three planes of signed base-256 digits;
+//   * W enters as the raw uint8 rows: TMA brings 128-column x 128-row boxes into shared memory in the layout the
+//     tensor core reads as a transposed (MN-major) operand, with no conversion and no thread touching a weight;
+//   * all sums are exact 32-bit integers (128 * 255 * K < 2^31 up to K = 65536), the planes and the K splits are
+//     combined in exact 64-bit integers and rounded to fp32 once: results do not depend on the tiling, on the split or
+//     on the form of the kernel.
+// W's 128 columns are the M side of the MMA and the tokens of all three planes its N side, so a launch of 16 tokens
+// multiplies 48 columns instead of padding 16 rows to 128.
+//
+// One persistent kernel: the tiles (matrix, column tile, token tile) are dealt in whole waves to the CTAs (or pairs of
+// CTAs, cta_group::2, sharing the token planes); the K range of the tiles left over is split so that they occupy the
+// whole GPU too.  A split tile is finished by the CTA that arrives last (tickets, no waiting), which adds the others'
+// 64-bit partial sums.
+//   warps 0-15 epilogue: tcgen05.ld of 32 TMEM lanes (warp % 4) x every fourth chunk of 8 tokens, affine tail and
+//              rounding into a shared-memory tile (the accumulators are free again), then the fused epilogue and the
+//              stores in 16-byte pieces of rows
+//   warp 16    TMEM allocation; tcgen05.mma and tcgen05.commit
+//   warp 17    TMA loads (W ahead of the dependency wait: it was written before the launch)
+// Every wait is bounded: on give-up the CTA raises an error word, skips the rest of its work and returns.
+#include "common.cuh"
+#include "seq_epi.cuh"
+#include <algorithm>
+#include <cuda.h>
+#include "mm8_seq_i8.h"
+
+namespace {
+
+constexpr int BMC = 128;                        // columns of W per CTA
+constexpr int BKI = 128;                        // K block
+constexpr int kWTile = BMC * BKI;               // 16 KB
+constexpr int kMaxTT = 128;                     // tokens per tile
+constexpr int kEpiThreads = 512;
+constexpr int kEpiWarps = kEpiThreads / 32;
+constexpr int kThreadsI8 = kEpiThreads + 64;
+constexpr int kMaxStages = 12;
+constexpr int kSmemBudget = 226 * 1024;
+constexpr unsigned kWaitLimitI8 = 1u << 22;
+constexpr float kTopDigits = 8355711.f;         // 127 * 65536 + 127 * 256 + 127
+
+struct alignas(16) RowConst { float scale, sx, sxr, sxmy; long long corr, pad; };      // corr = -128 * sum of the integers
+
+struct I8Problem {
+    const __half* mx; const __half* rx;
+    __half* y; long long y_stride;
+    SeqEpi epi;
+    int M, tile0;                               // tile0: index of this matrix's first tile
+    int vec;                                    // y, aux, aux2 allow 16-byte accesses
+};
+struct alignas(64) I8Args {
+    CUtensorMap wmap[kSeqI8MaxProblems];
+    CUtensorMap xmap[2];                        // the token planes as rows of 128 bytes, in boxes of the rows of each MMA
+    I8Problem p[kSeqI8MaxProblems];
+    const RowConst* consts;                     // [problem][T]
+    unsigned* tickets;                          // [split tile][CTA of the pair]
+    long long* slots;                           // [part of a split tile][CTA of the pair][TT][128]
+    unsigned* error_flag;
+    int nprob, T, TT, ntt, nkb, N1, N2, stages;
+    int units, whole, parts, split;             // unit u: tiles u, u + units, ... < whole, then part u (< parts) of the rest, `split` parts a tile
+    int bufcols;                                // TMEM columns between accumulator buffers (0: one buffer)
+    int tmem_cols;
+};
+
+__device__ __forceinline__ uint32_t su(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void bar_init(uint32_t b, uint32_t n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(b), "r"(n) : "memory"); }
+__device__ __forceinline__ void bar_arrive(uint32_t b) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(b) : "memory"); }
+__device__ __forceinline__ void bar_arrive_cluster(uint32_t b) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(b) : "memory");
+}
+__device__ __forceinline__ void bar_expect(uint32_t b, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(bytes) : "memory");
+}
+template <bool CLUSTER = false>                // CLUSTER: acquire what the other CTA of the pair released
+__device__ __forceinline__ bool bar_wait(uint32_t b, uint32_t parity) {
+    for (unsigned it = 0; it < kWaitLimitI8; ++it) {
+        uint32_t done;
+        if (CLUSTER)
+            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+                         "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(b), "r"(parity) : "memory");
+        else
+            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                         "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(b), "r"(parity) : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+// One lane of a converged warp.  The roles that issue MMAs and TMA loads run as whole warps and elect a lane for each
+// issue: descriptors then stay in uniform registers (issued from a lane == 0 branch, a K block cost 950 clocks).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
+}
+template <bool CLUSTER = false>                // the same answer in all lanes of a converged warp
+__device__ __forceinline__ bool warp_wait(uint32_t b, uint32_t parity) { return __all_sync(0xffffffffu, bar_wait<CLUSTER>(b, parity)); }
+__device__ __forceinline__ uint32_t in_cta(uint32_t local, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
+    return r;
+}
+// PAIR == 2: `bar` may be the barrier of the pair's first CTA, which counts the bytes of both
+template <int PAIR> __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+    if constexpr (PAIR == 2)
+        asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                     ::"r"(dst), "l"((uint64_t)map), "r"(x), "r"(y), "r"(bar) : "memory");
+    else
+        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                     ::"r"(dst), "l"((uint64_t)map), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+// Shared-memory matrix descriptor, 128-byte swizzle.  Both operands are stored as rows of 128 bytes whose 16-byte
+// chunks are permuted by (row % 8): for W a row is one k and its bytes are columns (MN-major), for the token planes a
+// row is one token and its bytes are k (K-major); 8-row groups follow each other at 1024 bytes.
+__device__ __forceinline__ uint64_t sw128_desc(uint32_t smem_addr) {
+    uint64_t d = (uint64_t)((smem_addr & 0x3FFFF) >> 4);
+    d |= (uint64_t)(1024 >> 4) << 16;
+    d |= (uint64_t)(1024 >> 4) << 32;
+    d |= (uint64_t)1 << 46;                     // descriptor version of sm_100
+    d |= (uint64_t)2 << 61;                     // 128-byte swizzle
+    return d;
+}
+// kind::i8: s32 accumulator, A unsigned 8 bit stored MN-major (transposed), B signed 8 bit stored K-major
+__device__ __forceinline__ uint32_t i8_idesc(int m, int n) {
+    return (2u << 4) | (0u << 7) | (1u << 10) | (1u << 15) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+}
+template <int PAIR>
+__device__ __forceinline__ void umma_i8(uint32_t d, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t accumulate) {
+    if constexpr (PAIR == 2)
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}"
+                     ::"r"(d), "l"(ad), "l"(bd), "r"(idesc), "r"(accumulate) : "memory");
+    else
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
+                     ::"r"(d), "l"(ad), "l"(bd), "r"(idesc), "r"(accumulate) : "memory");
+}
+template <int PAIR> __device__ __forceinline__ void commit_i8(uint32_t bar) {
+    if constexpr (PAIR == 2) {                  // the same barrier in both CTAs
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                     ::"r"(bar), "h"((uint16_t)3) : "memory");
+    } else {
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+    }
+}
+// fp32 of an exact 64-bit sum below 2^54, rounded once
+__device__ __forceinline__ float sum_to_f32(long long s) {
+    return fmaf((float)(int)(s >> 24), 16777216.f, (float)((int)s & 0xffffff));
+}
+// the fused epilogue on eight neighbouring columns (v already rounded to fp16: seq_epilogue_with starts from that)
+__device__ __forceinline__ void epi8(int mode, float scale, const __half (&v)[8], const __half (&x1)[8], const __half (&x2)[8], __half (&o)[8]) {
+    if (mode == RWKV_EPI_STORE) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) o[e] = v[e];
+    } else if (mode == RWKV_EPI_MUL_RESIDUAL || mode == RWKV_EPI_RESIDUAL) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) o[e] = seq_epilogue_with<__half>(mode, scale, __half2float(v[e]), __half2float(x1[e]), __half2float(x2[e]));
+    } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) o[e] = seq_epilogue_with<__half>(mode, scale, __half2float(v[e]), 0.f, 0.f);
+    }
+}
+__device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory"); }
+__device__ __forceinline__ void tmem_ld8(int (&v)[8], uint32_t addr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(addr) : "memory");
+}
+
+// ---- preparation: x' as digit planes, the row sums and scales ------------------------------------
+// One block per row (or per row and matrix); a thread owns a chunk of 16 k, kept in registers between the maximum and
+// the digits.
+__device__ __forceinline__ void load16(const __half* __restrict__ p, int k0, int N, bool vec, float (&out)[16]) {
+    if (vec && k0 + 16 <= N) {
+        const uint4 a = *reinterpret_cast<const uint4*>(p + k0), b = *reinterpret_cast<const uint4*>(p + k0 + 8);
+        const __half* ah = reinterpret_cast<const __half*>(&a);
+        const __half* bh = reinterpret_cast<const __half*>(&b);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) { out[e] = __half2float(ah[e]); out[8 + e] = __half2float(bh[e]); }
+    } else {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) out[e] = (k0 + e < N) ? __half2float(p[k0 + e]) : 0.f;
+    }
+}
+struct PrepProblem { const void* x; long long x_stride; const __half* ry; const __half* my; };
+struct PrepArgs {
+    PrepProblem p[kSeqI8MaxProblems];
+    int nprob, T, N, nkb, TT, ntt, ntickets, vec;          // vec: every vector and row starts on a 16-byte boundary
+    uint8_t* images; RowConst* consts; unsigned* tickets;
+};
+__device__ __forceinline__ void store_digits(const float (&xp)[16], float up, uint8_t* dst, size_t plane_bytes, int& isum) {
+    uint32_t d[3][4] = {};
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+        const int q = __float2int_rn(xp[e] * up);
+        isum += q;
+        const int d0 = (int)(int8_t)(q & 255), q1 = (q - d0) >> 8;
+        const int d1 = (int)(int8_t)(q1 & 255), d2 = (q1 - d1) >> 8;
+        d[0][e >> 2] |= (uint32_t)(d0 & 255) << (8 * (e & 3));
+        d[1][e >> 2] |= (uint32_t)(d1 & 255) << (8 * (e & 3));
+        d[2][e >> 2] |= (uint32_t)(d2 & 255) << (8 * (e & 3));
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i) *reinterpret_cast<uint4*>(dst + i * plane_bytes) = make_uint4(d[i][0], d[i][1], d[i][2], d[i][3]);
+}
+// Sums (MAX0: the first value's maximum) of NV values per thread over the block; every thread gets the results.
+template <int NV, bool MAX0>
+__device__ __forceinline__ void block_reduce(float (&v)[NV], float (*sh)[32]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) v[i] = (MAX0 && i == 0) ? warp_max(v[i]) : warp_sum(v[i]);
+    __syncthreads();                                       // the previous use of sh is over
+    if (lane == 0) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) sh[i][warp] = v[i];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        float t = sh[i][0];
+        for (int w = 1; w < nwarp; ++w) t = (MAX0 && i == 0) ? fmaxf(t, sh[i][w]) : t + sh[i][w];
+        v[i] = t;
+    }
+}
+
+// CH = 0: rows longer than 16384, read twice.
+template <int CH>
+__global__ void __launch_bounds__(1024) mm8_seq_i8_prep(const __grid_constant__ PrepArgs a) {
+    asm volatile("griddepcontrol.launch_dependents;");
+    const int t = blockIdx.x, tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarp = nthr >> 5;
+    __shared__ float sh[4][32];
+    __shared__ long long shq[32];
+    const bool vec = a.vec != 0;
+    const int N = a.N;
+    const int nchunk = a.nkb * (BKI / 16);
+    const bool mine = tid < nchunk;
+    float rv[16], mv[16];                                  // the first matrix's vectors do not depend on the work before
+    if (CH > 0 && mine) {
+        load16(a.p[blockIdx.y].ry, tid * 16, N, vec, rv);
+        load16(a.p[blockIdx.y].my, tid * 16, N, vec, mv);
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (t == 0 && blockIdx.y == 0)
+        for (int i = tid; i < a.ntickets; i += nthr) a.tickets[i] = 0;
+    // ---- digits, scale and sums for each matrix
+    const int tt = t / a.TT, ti = t - tt * a.TT;
+    const size_t plane = (size_t)a.TT * BKI;               // TT % 8 == 0: the three planes' rows share row % 8
+    for (int prob = blockIdx.y; prob < a.nprob; prob += gridDim.y) {
+        const PrepProblem& p = a.p[prob];
+        const __half* x = static_cast<const __half*>(p.x) + (long long)t * p.x_stride;
+        float xp[16] = {};
+        float red[4] = {0.f, 0.f, 0.f, 0.f};               // maximum, SX, SXR, SXMY
+        auto first = [&](int c) {
+            float xv[16];
+            load16(x, c * 16, N, vec, xv);
+            if (CH == 0 || prob != (int)blockIdx.y) {
+                load16(p.ry, c * 16, N, vec, rv);
+                load16(p.my, c * 16, N, vec, mv);
+            }
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+                xp[e] = xv[e] * rv[e];
+                red[1] += xv[e];
+                red[2] += xp[e];
+                red[3] = fmaf(xv[e], mv[e], red[3]);
+                red[0] = fabsf(xp[e]) <= 3.0e38f ? fmaxf(red[0], fabsf(xp[e])) : INFINITY;      // fmaxf would drop a NaN
+            }
+        };
+        if constexpr (CH > 0) { if (mine) first(tid); }
+        else for (int c = tid; c < nchunk; c += nthr) first(c);
+        block_reduce<4, true>(red, sh);
+        // the power of two `up` that takes the maximum into [2^22, 2^23), or half of it if three digits would not hold it
+        float up = 0.f, down = 0.f;
+        if (red[0] > 0.f && red[0] <= 3.0e38f) {
+            int e = 22 - ilogbf(red[0]);
+            if (ldexpf(red[0], e) > kTopDigits) --e;
+            up = ldexpf(1.f, e);                            // |x'| >= 2^-48 or 0: e <= 70
+            down = ldexpf(1.f, -e);
+        } else if (red[0] > 0.f) {
+            down = NAN;                                     // a NaN or an infinity among the activations: the row is NaN
+        }
+        const bool finite = down == down;
+        uint8_t* img = a.images + ((size_t)prob * a.ntt + tt) * a.nkb * (size_t)(3 * a.TT * BKI) + (size_t)ti * BKI;
+        auto second = [&](int c, int& isum) {
+            if (!finite) {
+#pragma unroll
+                for (int e = 0; e < 16; ++e) xp[e] = 0.f;
+            }
+            store_digits(xp, up, img + (size_t)(c >> 3) * (3 * plane) + (((c & 7) ^ (ti & 7)) << 4), plane, isum);
+        };
+        long long qsum = 0;
+        if constexpr (CH > 0) {
+            int isum = 0;
+            if (mine) second(tid, isum);
+            qsum = isum;
+        } else {
+            for (int c = tid; c < nchunk; c += nthr) {
+                float xv[16];
+                load16(x, c * 16, N, vec, xv);
+                load16(p.ry, c * 16, N, vec, rv);
+#pragma unroll
+                for (int e = 0; e < 16; ++e) xp[e] = xv[e] * rv[e];
+                int isum = 0;
+                second(c, isum);
+                qsum += isum;
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) qsum += __shfl_xor_sync(0xffffffffu, qsum, o);
+        __syncthreads();
+        if (lane == 0) shq[warp] = qsum;
+        __syncthreads();
+        if (tid == 0) {
+            RowConst rc;
+            rc.scale = down; rc.sx = red[1]; rc.sxr = red[2]; rc.sxmy = red[3]; rc.corr = 0; rc.pad = 0;
+            for (int i = 0; i < nwarp; ++i) rc.corr -= 128 * shq[i];
+            a.consts[(size_t)prob * a.T + t] = rc;
+        }
+    }
+}
+
+// ---- the matmul ------------------------------------------------------------------------------------
+struct Item { int prob, n0, tt, kb0, kb1, part; };        // part < 0: the whole K range
+// The i-th piece of work of `unit`; false when there is none.
+template <int PAIR> __device__ __forceinline__ bool item_of(const I8Args& a, int unit, int i, Item& t) {
+    int tile = unit + i * a.units;
+    t.kb0 = 0; t.kb1 = a.nkb; t.part = -1;
+    if (tile >= a.whole) {
+        if (unit >= a.parts || tile >= a.whole + a.units) return false;
+        const int r = unit / a.split, k = unit - r * a.split;
+        tile = a.whole + r;
+        if (a.split > 1) {
+            t.part = unit;
+            t.kb0 = a.nkb * k / a.split;
+            t.kb1 = a.nkb * (k + 1) / a.split;
+        }
+    }
+    t.prob = 0;
+#pragma unroll
+    for (int q = 1; q < kSeqI8MaxProblems; ++q) t.prob += (q < a.nprob && tile >= a.p[q].tile0) ? 1 : 0;
+    const int r = tile - a.p[t.prob].tile0, ct = r / a.ntt;
+    t.tt = r - ct * a.ntt;
+    t.n0 = ct * (BMC * PAIR);
+    return true;
+}
+
+template <int PAIR>
+__global__ void __launch_bounds__(kThreadsI8, 1) mm8_seq_i8_kernel(const __grid_constant__ I8Args a) {
+    asm volatile("griddepcontrol.launch_dependents;");
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = smem_raw + ((1024 - (su(smem_raw) & 1023)) & 1023);
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const uint32_t crank = PAIR == 2 ? (blockIdx.x & 1) : 0;
+    const int unit = blockIdx.x / PAIR;
+    const int S = a.stages;
+    const int n1 = a.N1 / PAIR, n2 = a.N2 / PAIR;                 // token rows of each MMA that this CTA holds
+    const uint32_t xbytes = (uint32_t)(n1 + n2) * BKI, stage_bytes = kWTile + xbytes;
+    uint8_t* bars = smem + (size_t)S * stage_bytes;
+    const uint32_t full0 = su(bars), empty0 = full0 + kMaxStages * 8;
+    const uint32_t acc_full0 = empty0 + kMaxStages * 8, acc_empty0 = acc_full0 + 16;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kMaxStages * 8 + 32);
+    volatile int* failed = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    int* last_flag = reinterpret_cast<int*>(tmem_slot + 2);
+    RowConst* rowc = reinterpret_cast<RowConst*>(bars + 512);     // [2][TT]
+    __half* tile = reinterpret_cast<__half*>(rowc + 2 * a.TT);    // [TT][128]: results before the fused epilogue
+
+    if (tid == 0) {
+        for (int s = 0; s < S; ++s) {
+            bar_init(full0 + s * 8, 1);
+            bar_init(empty0 + s * 8, 1);
+        }
+        for (int i = 0; i < 2; ++i) { bar_init(acc_full0 + i * 8, 1); bar_init(acc_empty0 + i * 8, kEpiWarps * PAIR); }
+        *failed = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == kEpiWarps) {
+        if constexpr (PAIR == 2) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su(tmem_slot)), "r"(a.tmem_cols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su(tmem_slot)), "r"(a.tmem_cols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    if constexpr (PAIR == 2) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    else __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp < kEpiWarps) {
+        // ================= epilogue =================
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        const int quarter = warp & 3, c_first = (warp >> 2) * 8;     // tokens c_first .. + 7, then 32 further on
+        bool ok = true;
+        Item tl;
+        for (int seg = 0; item_of<PAIR>(a, unit, seg, tl); ++seg) {
+            const I8Problem& p = a.p[tl.prob];
+            const bool whole = tl.part < 0;
+            const int buf = a.bufcols ? (seg & 1) : 0;
+            const uint32_t par = a.bufcols ? ((seg >> 1) & 1) : (seg & 1);
+            const int t0 = tl.tt * a.TT, n = tl.n0 + (int)crank * BMC + quarter * 32 + lane;
+            const int nlive = min(a.TT, a.T - t0);                    // tokens of this tile that exist
+            RowConst* rc = rowc + (seg & 1) * a.TT;
+            // row constants of this tile (its K loop is running meanwhile)
+            for (int i = tid; i < a.TT; i += kEpiThreads)
+                if (t0 + i < a.T) rc[i] = a.consts[(size_t)tl.prob * a.T + t0 + i];
+            const bool col = n < p.M;
+            const float rxn = col ? __half2float(p.rx[n]) : 0.f, mxn = col ? __half2float(p.mx[n]) : 0.f;
+            const float rx128 = rxn * 128.5f;
+            epi_sync();                                               // (and the previous tile's stores have left `tile`)
+            if (ok) ok = bar_wait(acc_full0 + buf * 8, par);
+            if (!ok) *failed = 1;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t tcol = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * a.bufcols);
+            long long* slot = whole ? nullptr : a.slots + (((size_t)tl.part * PAIR + crank) * a.TT) * BMC + quarter * 32 + lane;
+            __half* trow = tile + quarter * 32 + lane;
+            auto put = [&](int ti, long long s) {
+                const RowConst& r = rc[ti];
+                const float val = fmaf(rxn, sum_to_f32(s + r.corr) * r.scale, fmaf(rx128, r.sxr, fmaf(mxn, r.sx, r.sxmy)));
+                trow[ti * BMC] = __float2half_rn(val);
+            };
+            int q[2][3][8];                                           // the next chunk's loads run under this chunk's arithmetic
+            auto fetch = [&](int (&d)[3][8], int c) {
+#pragma unroll
+                for (int i = 0; i < 3; ++i) tmem_ld8(d[i], tcol + i * a.TT + c);
+            };
+            auto finish = [&](const int (&d)[3][8], int c) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const long long s = (long long)d[2][e] * 65536 + (long long)d[1][e] * 256 + d[0][e];
+                    if (whole) put(c + e, s);
+                    else if (c + e < nlive) slot[(size_t)(c + e) * BMC] = s;
+                }
+            };
+            if (c_first < nlive) fetch(q[0], c_first);
+#pragma unroll
+            for (int k = 0; k < kMaxTT / 32; ++k) {
+                const int c = c_first + 32 * k;
+                if (c >= nlive) break;
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (c + 32 < nlive) fetch(q[(k + 1) & 1], c + 32);
+                finish(q[k & 1], c);
+            }
+            // the accumulators are read: the next tile's MMAs may overwrite them
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) {
+                if (PAIR == 2) bar_arrive_cluster(in_cta(acc_empty0 + buf * 8, 0));
+                else bar_arrive(acc_empty0 + buf * 8);
+            }
+            if (!whole) {
+                const int r = tl.part / a.split;                       // split tile
+                __threadfence();
+                epi_sync();
+                if (tid == 0) *last_flag = ok && atomicAdd(a.tickets + (size_t)r * PAIR + crank, 1u) == (unsigned)(a.split - 1);
+                epi_sync();
+                if (*last_flag == 0) continue;
+                __threadfence();
+                // two neighbouring columns per thread and step, 16 loads in flight
+                const size_t part_stride = (size_t)PAIR * a.TT * BMC / 2;
+                const longlong2* first = reinterpret_cast<const longlong2*>(a.slots + ((size_t)r * a.split * PAIR + crank) * a.TT * BMC);
+                const int n2c = tl.n0 + (int)crank * BMC + (tid & 63) * 2, end = min(a.TT, a.T - t0) * (BMC / 2);
+                const bool c0 = n2c < p.M, c1 = n2c + 1 < p.M;
+                const float rx0 = c0 ? __half2float(p.rx[n2c]) : 0.f, mx0 = c0 ? __half2float(p.mx[n2c]) : 0.f;
+                const float rx1 = c1 ? __half2float(p.rx[n2c + 1]) : 0.f, mx1 = c1 ? __half2float(p.mx[n2c + 1]) : 0.f;
+                for (int i = tid; i < end; i += 4 * kEpiThreads) {
+                    longlong2 s[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) { const long long cr = rc[min(i + q * kEpiThreads, end - 1) >> 6].corr; s[q] = make_longlong2(cr, cr); }
+#pragma unroll 4
+                    for (int u = 0; u < a.split; ++u) {
+                        longlong2 l[4];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            l[q] = i + q * kEpiThreads < end ? __ldcg(first + u * part_stride + i + q * kEpiThreads) : make_longlong2(0, 0);
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) { s[q].x += l[q].x; s[q].y += l[q].y; }
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int j = i + q * kEpiThreads;
+                        if (j >= end) break;
+                        const RowConst& k = rc[j >> 6];
+                        const float v0 = fmaf(rx0, sum_to_f32(s[q].x) * k.scale, fmaf(rx0 * 128.5f, k.sxr, fmaf(mx0, k.sx, k.sxmy)));
+                        const float v1 = fmaf(rx1, sum_to_f32(s[q].y) * k.scale, fmaf(rx1 * 128.5f, k.sxr, fmaf(mx1, k.sx, k.sxmy)));
+                        reinterpret_cast<__half2*>(tile)[j] = __halves2half2(__float2half_rn(v0), __float2half_rn(v1));
+                    }
+                }
+            }
+            epi_sync();                                               // the tile of results is complete
+            if (!ok) continue;
+            const int mode = p.epi.mode, M = p.M, nb = tl.n0 + (int)crank * BMC, tlive = min(a.TT, a.T - t0);
+            const float scale = p.epi.out_scale;
+            const bool has1 = mode == RWKV_EPI_RESIDUAL || mode == RWKV_EPI_MUL_RESIDUAL, has2 = mode == RWKV_EPI_MUL_RESIDUAL;
+            __half* y = p.y + (long long)t0 * p.y_stride;
+            const __half* x1p = static_cast<const __half*>(p.epi.aux) + (has1 ? (long long)t0 * p.epi.aux_stride : 0);
+            const __half* x2p = static_cast<const __half*>(p.epi.aux2) + (has2 ? (long long)t0 * p.epi.aux2_stride : 0);
+            const long long ys = p.y_stride, s1 = p.epi.aux_stride, s2 = p.epi.aux2_stride;
+            const bool vec = p.vec != 0;
+#pragma unroll 2
+            for (int i = tid; i < tlive * (BMC / 8); i += kEpiThreads) {
+                const int t = i >> 4, nn = nb + (i & 15) * 8, live = M - nn;
+                if (live <= 0) continue;
+                __half v[8], x1[8] = {}, x2[8] = {}, o[8];
+                *reinterpret_cast<uint4*>(v) = *reinterpret_cast<const uint4*>(tile + t * BMC + (i & 15) * 8);
+                if (vec && live >= 8) {
+                    if (has1) *reinterpret_cast<uint4*>(x1) = *reinterpret_cast<const uint4*>(x1p + t * s1 + nn);
+                    if (has2) *reinterpret_cast<uint4*>(x2) = *reinterpret_cast<const uint4*>(x2p + t * s2 + nn);
+                    epi8(mode, scale, v, x1, x2, o);
+                    *reinterpret_cast<uint4*>(y + t * ys + nn) = *reinterpret_cast<const uint4*>(o);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        if (e < live) {
+                            if (has1) x1[e] = x1p[t * s1 + nn + e];
+                            if (has2) x2[e] = x2p[t * s2 + nn + e];
+                        }
+                    epi8(mode, scale, v, x1, x2, o);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        if (e < live) y[t * ys + nn + e] = o[e];
+                }
+            }
+        }
+    } else if (warp == kEpiWarps + 1) {
+        // ================= TMA loads =================
+        {
+            bool ok = true;
+            int s = 0;
+            uint32_t ph = 1;                                           // the stages start empty
+            const uint32_t smem0 = su(smem);
+            const int xrows = 3 * a.TT;                                // rows of one K block of the token planes
+            auto full_of = [&](int st) { return PAIR == 2 ? in_cta(full0 + st * 8, 0) : full0 + st * 8; };
+            Item tl;
+            for (int seg = 0; ok && item_of<PAIR>(a, unit, seg, tl); ++seg) {
+                const CUtensorMap* map = &a.wmap[tl.prob];
+                const int n0 = tl.n0 + (int)crank * BMC, nb = tl.kb1 - tl.kb0;
+                int row = ((tl.prob * a.ntt + tl.tt) * a.nkb + tl.kb0) * xrows;
+                auto load_w = [&](int i, int st) {
+                    if (elect_one()) {
+                        if (crank == 0) bar_expect(full0 + st * 8, PAIR * stage_bytes);
+                        tma_load_2d<PAIR>(smem0 + st * stage_bytes, map, n0, (tl.kb0 + i) * BKI, full_of(st));
+                    }
+                };
+                auto load_x = [&](int st) {
+                    const uint32_t dst = smem0 + st * stage_bytes + kWTile;
+                    if (elect_one()) {
+                        tma_load_2d<PAIR>(dst, &a.xmap[0], 0, row + (int)crank * n1, full_of(st));
+                        if (n2) tma_load_2d<PAIR>(dst + n1 * BKI, &a.xmap[1], 0, row + a.N1 + (int)crank * n2, full_of(st));
+                    }
+                    row += xrows;
+                };
+                int i = 0;
+                if (seg == 0) {                                        // W does not depend on the work before this launch
+                    const int ahead = min(S, nb);
+                    for (; i < ahead; ++i) load_w(i, i);
+                    asm volatile("griddepcontrol.wait;" ::: "memory");
+                    asm volatile("fence.proxy.async;" ::: "memory");   // the planes were written by ordinary stores
+                    for (int q = 0; q < ahead; ++q) load_x(q);
+                    s = ahead == S ? 0 : ahead;
+                    ph = ahead == S ? 0u : 1u;
+                }
+                for (; i < nb; ++i) {
+                    ok = warp_wait(empty0 + s * 8, ph);
+                    if (!ok) break;
+                    load_w(i, s);
+                    load_x(s);
+                    if (++s == S) { s = 0; ph ^= 1; }
+                }
+            }
+            if (!ok) *failed = 1;
+        }
+    } else if (crank == 0) {
+        // ================= MMA issuer =================
+        const uint32_t id1 = i8_idesc(BMC * PAIR, a.N1), id2 = i8_idesc(BMC * PAIR, a.N2 ? a.N2 : a.N1);
+        bool ok = true;
+        int s = 0;
+        uint32_t ph = 0;
+        const uint64_t ad0 = sw128_desc(su(smem)), xd0 = sw128_desc(su(smem) + kWTile);
+        Item tl;
+        for (int seg = 0; ok && item_of<PAIR>(a, unit, seg, tl); ++seg) {
+            const int nb = tl.kb1 - tl.kb0;
+            const int buf = a.bufcols ? (seg & 1) : 0;
+            const uint32_t par = a.bufcols ? ((seg >> 1) & 1) : (seg & 1);
+            ok = warp_wait<PAIR == 2>(acc_empty0 + buf * 8, par ^ 1);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t d = tmem + (uint32_t)(buf * a.bufcols);
+            for (int i = 0; i < nb && ok; ++i) {
+                ok = warp_wait(full0 + s * 8, ph);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint64_t ad = ad0 + ((uint32_t)s * stage_bytes >> 4), xd = xd0 + ((uint32_t)s * stage_bytes >> 4);
+                if (elect_one()) {
+#pragma unroll
+                    for (int j = 0; j < BKI / 32; ++j) {           // one UMMA consumes K = 32: 32 rows of W, 32 bytes of the planes
+                        const uint32_t acc = (i > 0 || j > 0) ? 1u : 0u;
+                        umma_i8<PAIR>(d, ad + (j * 32 * 128 >> 4), xd + (j * 32 >> 4), id1, acc);
+                        if (n2) umma_i8<PAIR>(d + a.N1, ad + (j * 32 * 128 >> 4), xd + ((n1 * BKI + j * 32) >> 4), id2, acc);
+                    }
+                    commit_i8<PAIR>(empty0 + s * 8);
+                }
+                __syncwarp();
+                if (++s == S) { s = 0; ph ^= 1; }
+            }
+            if (ok && elect_one()) commit_i8<PAIR>(acc_full0 + buf * 8);
+            __syncwarp();
+        }
+        if (!ok) *failed = 1;
+    }
+
+    __syncwarp();
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    if constexpr (PAIR == 2) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    else __syncthreads();
+    if (*failed) {                                                 // a wait gave up: give copies still in flight time to land
+        for (int i = 0; i < 64; ++i) __nanosleep(1000);
+        __syncthreads();
+    }
+    if (warp == kEpiWarps) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if constexpr (PAIR == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(a.tmem_cols) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(a.tmem_cols) : "memory");
+    }
+    if (tid == 0 && *failed) atomicExch(a.error_flag, 1u);
+}
+
+// ---- host side -------------------------------------------------------------------------------------
+struct Plan {
+    int TT, ntt, nkb, pair, N1, N2, stages, smem, units, whole, parts, split, ntiles, bufcols, tmem_cols;
+    size_t tickets, consts, images, slots, bytes;                 // offsets in the workspace, its size
+};
+
+// Estimated time of a tile whose K blocks are dealt to `k` CTAs, `ctas` of them at work: a block takes the tensor cores
+// 0.28 us (0.39 us with 128 tokens) and HBM 16 KB per CTA; parts cost the exchange through L2.
+double split_cost_us(int nkb, int k, int TT, int ctas) {
+    const double block = std::max(std::max(0.28, 0.39 * TT / 128), 0.0025 * ctas);
+    return (nkb + k - 1) / k * block + (k > 1 ? 2.5 + 0.02 * TT + 0.1 * k : 0.0);
+}
+
+Plan make_plan(int nprob, int64_t T, int64_t N, const int64_t* M, int force) {
+    Plan p;
+    const int sms = rwkv_sm_count();
+    p.nkb = int((N + BKI - 1) / BKI);
+    p.ntt = int((T + kMaxTT - 1) / kMaxTT);
+    const int per = int((T + p.ntt - 1) / p.ntt);
+    p.pair = force == 1 ? 0 : force == 2 ? 1 : (per > 32 ? 1 : 0);
+    const int unit = p.pair ? 32 : 16;
+    p.TT = (per + unit - 1) / unit * unit;
+    const int n = 3 * p.TT;
+    p.N1 = n <= 256 ? n : (n / 2 + unit - 1) / unit * unit;
+    p.N2 = n - p.N1;
+    const int pc = p.pair ? 2 : 1;
+    const int stage = kWTile + n / pc * BKI;
+    const int tail = 512 + p.TT * (2 * int(sizeof(RowConst)) + BMC * 2);
+    p.stages = std::min(kMaxStages, (kSmemBudget - 1024 - tail) / stage);
+    p.smem = 1024 + p.stages * stage + tail;
+    p.bufcols = n <= 256 ? 256 : 0;
+    p.tmem_cols = 512;
+    p.ntiles = 0;
+    for (int i = 0; i < nprob; ++i) p.ntiles += int((M[i] + BMC * pc - 1) / (BMC * pc)) * p.ntt;
+    // whole waves, then the rest split along K (at least two K blocks a part) over the units
+    const int umax = sms / pc;
+    p.whole = p.ntiles / umax * umax;
+    const int rest = p.ntiles - p.whole;
+    p.split = 1;
+    double best = 1e30;
+    for (int k = 1; rest > 0 && k <= std::max(1, std::min(umax / rest, p.nkb / 2)); ++k) {
+        const double t = split_cost_us(p.nkb, k, p.TT, rest * k * pc);
+        if (t < best) { best = t; p.split = k; }
+    }
+    p.parts = rest * p.split;
+    p.units = p.whole > 0 ? umax : p.parts;
+    auto up = [](size_t v) { return (v + 1023) / 1024 * 1024; };
+    p.tickets = 1024;
+    p.consts = up(p.tickets + size_t(umax) * pc * 4);
+    p.images = up(p.consts + size_t(nprob) * T * sizeof(RowConst));
+    p.slots = up(p.images + size_t(nprob) * p.ntt * p.nkb * size_t(n) * BKI);
+    p.bytes = p.slots + (p.split > 1 ? size_t(p.parts) * pc * p.TT * BMC * 8 : 0);
+    return p;
+}
+
+typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                             const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeFn encode_fn() {
+    static EncodeFn fn = []() -> EncodeFn {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult st;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &st) != cudaSuccess || st != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        return reinterpret_cast<EncodeFn>(f);
+    }();
+    return fn;
+}
+
+int g_i8_form = 0;                       // 0 automatic, 1 one CTA per tile, 2 pairs (set through rwkv_mm8_seq_set_path)
+
+}  // namespace
+
+void rwkv_mm8_seq_i8_set_form(int form) { g_i8_form = form; }
+
+size_t rwkv_mm8_seq_i8_workspace_bytes(int nprob, int64_t T, int64_t N, const int64_t* M) {
+    if (nprob < 1 || nprob > kSeqI8MaxProblems || T < 1 || N < 1 || N > 65536) return 0;
+    return std::max(make_plan(nprob, T, N, M, 1).bytes, make_plan(nprob, T, N, M, 2).bytes);
+}
+
+int rwkv_mm8_seq_i8(int nprob, const SeqI8Problem* probs, int64_t T, int64_t N, void* workspace, size_t workspace_bytes, void* stream) {
+    RWKV_CHECK_ARG(nprob >= 1 && nprob <= kSeqI8MaxProblems && T >= 1 && N >= 1);
+    if (N > 65536 || T > (1 << 18)) return RWKV_ERR_UNSUPPORTED;
+    int64_t M[kSeqI8MaxProblems];
+    for (int i = 0; i < nprob; ++i) {
+        const SeqI8Problem& q = probs[i];
+        if (reinterpret_cast<uintptr_t>(q.w) % 16 != 0 || q.w_stride % 16 != 0) return RWKV_ERR_UNSUPPORTED;   // TMA rows
+        M[i] = q.M;
+    }
+    if (encode_fn() == nullptr) return RWKV_ERR_UNSUPPORTED;
+    const Plan p = make_plan(nprob, T, N, M, g_i8_form);
+    if (workspace == nullptr || workspace_bytes < p.bytes) return RWKV_ERR_WORKSPACE;
+    RWKV_CHECK_ALIGN(workspace, 256);
+    uint8_t* ws = static_cast<uint8_t*>(workspace);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+
+    I8Args a;
+    memset(&a, 0, sizeof(a));
+    PrepArgs pa;
+    memset(&pa, 0, sizeof(pa));
+    const int pc = p.pair ? 2 : 1;
+    int tile = 0;
+    bool vec = true;
+    auto al = [](const void* ptr, int64_t stride_bytes) { return reinterpret_cast<uintptr_t>(ptr) % 16 == 0 && stride_bytes % 16 == 0; };
+    for (int i = 0; i < nprob; ++i) {
+        const SeqI8Problem& q = probs[i];
+        const cuuint64_t dims[2] = {(cuuint64_t)q.M, (cuuint64_t)N}, strides[1] = {(cuuint64_t)q.w_stride};
+        const cuuint32_t box[2] = {BMC, BKI}, es[2] = {1, 1};
+        if (encode_fn()(&a.wmap[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(q.w), dims, strides, box, es,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return RWKV_ERR_UNSUPPORTED;
+        I8Problem& d = a.p[i];
+        d.mx = static_cast<const __half*>(q.mx); d.rx = static_cast<const __half*>(q.rx);
+        d.vec = al(q.y, q.y_stride * 2) && (q.epi.aux == nullptr || al(q.epi.aux, q.epi.aux_stride * 2)) &&
+                (q.epi.aux2 == nullptr || al(q.epi.aux2, q.epi.aux2_stride * 2));
+        d.y = static_cast<__half*>(q.y); d.y_stride = q.y_stride; d.epi = q.epi; d.M = int(q.M); d.tile0 = tile;
+        tile += int((q.M + BMC * pc - 1) / (BMC * pc)) * p.ntt;
+        PrepProblem& r = pa.p[i];
+        r.x = q.x; r.x_stride = q.x_stride;
+        r.ry = static_cast<const __half*>(q.ry); r.my = static_cast<const __half*>(q.my);
+        vec = vec && al(q.x, q.x_stride * 2) && al(q.ry, 0) && al(q.my, 0);
+    }
+    pa.nprob = nprob; pa.vec = vec ? 1 : 0; pa.T = int(T); pa.N = int(N); pa.nkb = p.nkb; pa.TT = p.TT; pa.ntt = p.ntt;
+    pa.ntickets = p.split > 1 ? p.parts / p.split * pc : 0;
+    pa.images = ws + p.images; pa.consts = reinterpret_cast<RowConst*>(ws + p.consts); pa.tickets = reinterpret_cast<unsigned*>(ws + p.tickets);
+    const long long xrows = (long long)nprob * p.ntt * p.nkb * 3 * p.TT;
+    if (xrows >= (1ll << 31)) return RWKV_ERR_UNSUPPORTED;
+    for (int i = 0; i < (p.N2 ? 2 : 1); ++i) {
+        const cuuint64_t dims[2] = {BKI, (cuuint64_t)xrows}, strides[1] = {BKI};
+        const cuuint32_t box[2] = {BKI, (cuuint32_t)((i ? p.N2 : p.N1) / pc)}, es[2] = {1, 1};
+        if (encode_fn()(&a.xmap[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, pa.images, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return RWKV_ERR_UNSUPPORTED;
+    }
+    a.consts = pa.consts; a.tickets = pa.tickets; a.slots = reinterpret_cast<long long*>(ws + p.slots);
+    a.error_flag = reinterpret_cast<unsigned*>(ws);
+    a.nprob = nprob; a.T = int(T); a.TT = p.TT; a.ntt = p.ntt; a.nkb = p.nkb; a.N1 = p.N1; a.N2 = p.N2; a.stages = p.stages;
+    a.units = p.units; a.whole = p.whole; a.parts = p.parts; a.split = p.split;
+    a.bufcols = p.bufcols; a.tmem_cols = p.tmem_cols;
+
+    static bool configured[64] = {};         // function attributes are per device
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) { cudaGetLastError(); return RWKV_ERR_LAUNCH; }
+    if (dev >= 64 || !configured[dev]) {
+        if (cudaFuncSetAttribute(mm8_seq_i8_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget) != cudaSuccess ||
+            cudaFuncSetAttribute(mm8_seq_i8_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget) != cudaSuccess) {
+            cudaGetLastError();
+            return RWKV_ERR_LAUNCH;
+        }
+        if (dev < 64) configured[dev] = true;
+    }
+    const int nchunk = p.nkb * (BKI / 16);
+    const int threads = std::min(1024, (nchunk + 31) / 32 * 32);
+    // few rows: a block per (row, matrix), so that they run side by side; many: a block per row
+    const dim3 pgrid((unsigned)T, (unsigned)(T * nprob <= 2 * rwkv_sm_count() ? nprob : 1));
+    int rc = nchunk <= 1024 ? rwkv_launch_pdl(mm8_seq_i8_prep<1>, pgrid, dim3(threads), 0, st, pa)
+                            : rwkv_launch_pdl(mm8_seq_i8_prep<0>, pgrid, dim3(threads), 0, st, pa);
+    if (rc != RWKV_OK) return rc;
+    if (!p.pair) return rwkv_launch_pdl(mm8_seq_i8_kernel<1>, dim3(p.units), dim3(kThreadsI8), size_t(p.smem), st, a);
+    return rwkv_launch_pdl_clustered(2, mm8_seq_i8_kernel<2>, dim3(p.units * 2), dim3(kThreadsI8), size_t(p.smem), st, a);
+}

@@ -1,4 +1,6 @@
-// mm8_seq on the 5th-generation tensor cores (tcgen05, accumulators in tensor memory).
+// mm8_seq on the fp16 path of the 5th-generation tensor cores (tcgen05, accumulators in tensor memory): the form for
+// packed matrices whose rows TMA cannot fetch (8-byte instead of 16-byte alignment) and for the single-pass option;
+// mm8_seq_i8.cu runs everything else.
 //
 //   y[t,n] = rx[n] * sum_k x'[t,k] (w[k,n] - 128) + rx[n]*128.5*SXR[t] + mx[n]*SX[t] + SXMY[t]
 //

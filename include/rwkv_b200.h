@@ -328,16 +328,17 @@ int rwkv_mm8_stream_take_error(uint32_t* sync_words, void* stream, int* error_ou
  *
  * x [B, N] row stride x_stride, y [B, M] row stride y_stride, both in `dtype`, fp32
  * accumulation, one rounding to `dtype` at the store (operators.cu:138).
- * Two kernels: from 8 rows up, fp16 operands whose w is 8-byte aligned (pointer, stride, M)
- * run on the tensor cores (tcgen05 UMMA, fp32 accumulation in tensor memory; x*ry enters as
- * an exact hi + lo pair of fp16 values) and need `workspace` =
- * rwkv_mm8_seq_workspace_bytes(B, N, M) bytes, 256-byte aligned, zero when first handed over;
+ * Three kernels.  From 2 rows up, fp16 operands whose w rows are 16-byte aligned (pointer, stride; any M, N up
+ * to 65536) run on the integer path of the tensor cores (tcgen05 kind::i8, csrc/mm8_seq_i8.cu): the bytes of w
+ * as they are, x*ry as 24-bit fixed point per row in three base-256 digits, exact integer sums; results do not
+ * depend on the tiling.  From 8 rows up, w that is only 8-byte aligned (pointer, stride, M) runs on the fp16 path
+ * (kind::f16, csrc/mm8_seq_tc.cu; x*ry enters as an exact hi + lo pair of fp16 values).  Both need
+ * `workspace` = rwkv_mm8_seq_workspace_bytes(B, N, M) bytes, 256-byte aligned, zero when first handed over;
  * everything else (or workspace == NULL) runs on a CUDA-core kernel that accepts any layout.
  * rwkv_mm8_seq_set_path: 0 automatic, 1 CUDA cores only, 2 tensor cores whenever possible; adding 4
- * makes the tensor-core kernel multiply fp16(x*ry) in ONE pass instead of the exact hi + lo pair
- * (about 1e-4 of the output's RMS less accurate, 10-35 % faster at T = 1024; off by default); adding 8
- * keeps one CTA per output tile (by default launches with an even number of 128-row tiles and no K
- * split run as clusters of two CTAs sharing one 256-row UMMA, tcgen05 cta_group::2; same results).
+ * multiplies fp16(x*ry) in ONE pass of the fp16 path (about 1e-4 of the output's RMS less accurate, and
+ * slower than the exact integer path; kept for programs that set it); adding 8 keeps one CTA per output tile (by
+ * default larger launches run as clusters of two CTAs sharing one 256-row UMMA, tcgen05 cta_group::2; same results).
  * rwkv_mm8_seq_tc_take_error synchronises `stream` and returns/clears the workspace's error
  * word (1 if a bounded wait inside the tensor-core kernel gave up; outputs then undefined).
  * ------------------------------------------------------------------------------------- */

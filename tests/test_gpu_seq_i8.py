@@ -1,0 +1,83 @@
+"""mm8_seq on tcgen05 kind::i8 (csrc/mm8_seq_i8.cu): the edges of its tiles, K blocks, splits and forms."""
+import ctypes
+
+import pytest
+import torch
+
+from oracle import rwkv_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from chatrwkv_b200 import ops as o
+    return o
+
+
+def _error_word(ops):
+    from chatrwkv_b200 import _lib
+    ws = ops.workspace(torch.device("cuda", torch.cuda.current_device()), 1024, "mm8_seq")
+    e = ctypes.c_int(-1)
+    assert _lib.lib().rwkv_mm8_seq_tc_take_error(ws.data_ptr(), None, ctypes.byref(e)) == 0
+    return e.value
+
+
+# rows around the tile sizes (16 / 32 up to 128) and the one-CTA / CTA-pair boundary, in-features around the K block of 128
+# and past the one-chunk-per-thread preparation, out-features that are no multiple of 8 or 128, and more tiles than CTAs
+@pytest.mark.parametrize("T,N,M", [(2, 16, 8), (15, 127, 277), (16, 128, 128), (17, 129, 129), (32, 640, 4096), (33, 4096, 1000),
+                                   (64, 2048, 256), (65, 300, 50277), (96, 256, 2304), (127, 1024, 640), (129, 512, 384),
+                                   (300, 384, 9000), (3, 16400, 200), (40, 20480, 136)])
+def test_edges_against_oracle_and_one_cta_form(ops, T, N, M):
+    from chatrwkv_b200 import _lib
+    from tests.util import packed_case
+    cpu, dev = packed_case(N, M, seed=T + N + M)
+    g = torch.Generator().manual_seed(T)
+    x = torch.randn(T, N, generator=g).half()
+    y = torch.full((T, M), float("nan"), dtype=torch.float16, device="cuda")
+    torch.ops.rwkv.mm8_seq(T, N, M, x.cuda(), *dev, y)
+    _lib.lib().rwkv_mm8_seq_set_path(8)
+    try:
+        y1 = torch.full((T, M), float("nan"), dtype=torch.float16, device="cuda")
+        torch.ops.rwkv.mm8_seq(T, N, M, x.cuda(), *dev, y1)
+    finally:
+        _lib.lib().rwkv_mm8_seq_set_path(0)
+    torch.cuda.synchronize()
+    assert _error_word(ops) == 0
+    assert torch.equal(y, y1)                       # exact integer sums: no dependence on the form or the K split
+    ref = orc.mm8_kernel(x, *cpu)
+    # one rounding to fp16 (2^-11 relative), and fp32 terms of a few times the result's size
+    assert ((y.float().cpu() - ref).abs() <= ref.abs() * 2 ** -10 + 1e-4).all()
+
+
+def test_non_finite_rows_stay_in_their_row(ops):
+    from tests.util import packed_case
+    T, N, M = 40, 512, 300
+    cpu, dev = packed_case(N, M, seed=2)
+    x = torch.randn(T, N, generator=torch.Generator().manual_seed(3)).half()
+    ref = orc.mm8_kernel(x, *cpu)
+    bad = x.clone()
+    bad[5, 17], bad[33, 500] = float("nan"), float("-inf")
+    bad[7] = 0
+    y = torch.empty((T, M), dtype=torch.float16, device="cuda")
+    torch.ops.rwkv.mm8_seq(T, N, M, bad.cuda(), *dev, y)
+    y = y.float().cpu()
+    assert not torch.isfinite(y[[5, 33]]).any()
+    assert (y[7] == 0).all()
+    rest = [t for t in range(T) if t not in (5, 7, 33)]
+    assert ((y[rest] - ref[rest]).abs() <= ref[rest].abs() * 2 ** -10 + 1e-4).all()
+
+
+@pytest.mark.parametrize("magnitude", [6e-8, 1e-3, 3e4])
+def test_range_of_the_fixed_point_scale(ops, magnitude):
+    """The power-of-two scale follows the row: subnormal and huge activations keep their relative accuracy."""
+    from tests.util import packed_case
+    T, N, M = 16, 256, 128
+    cpu, dev = packed_case(N, M, seed=4)
+    x = (torch.randn(T, N, generator=torch.Generator().manual_seed(5)).clamp(-2, 2) * magnitude).half()
+    ref = orc.mm8_kernel(x, *cpu)
+    y = torch.empty((T, M), dtype=torch.float16, device="cuda")
+    torch.ops.rwkv.mm8_seq(T, N, M, x.cuda(), *dev, y)
+    scale = ref.abs().max().item()
+    ok = (y.float().cpu() - ref.half().float()).abs() <= ref.abs() * 2 ** -10 + max(scale * 1e-5, 6e-8)
+    assert ok[ref.abs() < 6e4].all()
