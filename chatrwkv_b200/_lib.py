@@ -16,6 +16,7 @@ F32, F16, BF16 = 0, 1, 2
 PRO_PLAIN, PRO_LN_MIX, PRO_WKV4 = 0, 1, 2
 ERR_UNSUPPORTED = -5
 MM8_WIDE_BUILD = 1
+SEQ_F16_SUMS = 0x100      # added to an epilogue of mm8_seq_epi
 EPI_ACC_F32, EPI_STORE, EPI_SIGMOID, EPI_RELU_SQ, EPI_RESIDUAL, EPI_MUL_RESIDUAL, EPI_STORE_F32, EPI_SILU = range(8)
 
 

@@ -135,11 +135,13 @@ extern "C" int rwkv_mm8_seq_epi(int64_t B, int64_t N, int64_t M, const void* x, 
     RWKV_CHECK_ARG(x && w && mx && rx && my && ry && y);
     RWKV_CHECK_ARG(x_stride >= N && w_stride >= M && y_stride >= M);
     RWKV_CHECK_ARG(dtype == RWKV_F16 || dtype == RWKV_F32);
+    const bool f16_sums = (epilogue & RWKV_SEQ_F16_SUMS) != 0;
+    epilogue &= ~RWKV_SEQ_F16_SUMS;
     SeqEpi epi;
     epi.mode = epilogue; epi.out_scale = out_scale; epi.aux = aux; epi.aux_stride = aux_stride; epi.aux2 = aux2; epi.aux2_stride = aux2_stride;
     const int erc = seq_epi_check(epi);
     if (erc != RWKV_OK) return erc;
-    if (g_seq_path != 1 && !g_seq_single && workspace != nullptr && dtype == RWKV_F16 && (B >= kI8MinRows || g_seq_path == 2)) {
+    if (g_seq_path != 1 && !g_seq_single && !f16_sums && workspace != nullptr && dtype == RWKV_F16 && (B >= kI8MinRows || g_seq_path == 2)) {
         const SeqI8Problem p = {x, x_stride, w, w_stride, mx, rx, my, ry, y, y_stride, M, epi};
         const int rc = rwkv_mm8_seq_i8(1, &p, B, N, workspace, workspace_bytes, stream);
         if (rc != RWKV_ERR_UNSUPPORTED && rc != RWKV_ERR_WORKSPACE) return rc;   // else: the general kernels below

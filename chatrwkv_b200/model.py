@@ -412,7 +412,8 @@ class RWKV:
 
     def forward(self, tokens, state, full_output=False):
         with torch.no_grad(), torch.cuda.device(self.device):
-            if state is None:
+            fresh = state is None
+            if fresh:
                 state = self._zero_state()
             if torch.is_tensor(tokens):
                 if tokens.is_cuda and tokens.numel() == 1 and self._all_i8:
@@ -420,7 +421,7 @@ class RWKV:
                 tokens = tokens.tolist()
             if len(tokens) == 1 and self._all_i8:
                 return self._forward_one(int(tokens[0]), state)
-            return self._forward_seq([int(t) for t in tokens], state, full_output)
+            return self._forward_seq([int(t) for t in tokens], state, full_output, fresh)
 
     # ----- one token ---------------------------------------------------------------------
     @property
@@ -865,10 +866,13 @@ class RWKV:
             torch.ops.rwkv.mm8_seq(T, N, M, x, wq, mx, rx, my, ry, y)
         return y if out_dtype is None else y.to(out_dtype)
 
-    def _mm_epi(self, x, name, epilogue, aux=None, aux2=None, out_scale=1.0, out=None):
-        """mm8_seq with the reference's next pointwise op(s) fused into the store (single-GPU path)."""
+    def _mm_epi(self, x, name, epilogue, aux=None, aux2=None, out_scale=1.0, out=None, early=False):
+        """mm8_seq with the reference's next pointwise op(s) fused into the store (single-GPU path).  `early`: see
+        EARLY_PROMPT."""
         if self.w[name].dtype != torch.uint8:
             return self._plain(x, name, epilogue, aux, aux2, out_scale, out)
+        if early:
+            epilogue |= _lib.SEQ_F16_SUMS
         wq, mx, rx, my, ry = self._scales(name)
         M = wq.shape[1]
         if M % 8 != 0 and out is None and aux is None and aux2 is None and wq.stride(0) >= (M + 7) // 8 * 8:
@@ -953,7 +957,7 @@ class RWKV:
         st[i * 5 + 0] = new_sx
         return x + out
 
-    def _att_seq_v56(self, x, st2, i, rows=False):
+    def _att_seq_v56(self, x, st2, i, rows=False, early=False):
         """cuda_att_seq_v5_2 / cuda_att_seq_v6_0 (model.py:1363-1439).  `st2` = [att_xx, att_kv]; the first entry is
         replaced, the matrix state is updated in place in the model's [H, key, value] layout.  Kernels of this
         library throughout; the four small low-rank products of RWKV-6 (ranks 32..160) are plain fp16 library GEMMs
@@ -1014,10 +1018,10 @@ class RWKV:
                                         (vx, att + "value.weight", EPI_STORE), (gx, att + "gate.weight", EPI_SILU)],
                                        extra=decay_chain if self.version == 6 else None)
         else:
-            r = self._mm_epi(rx, att + "receptance.weight", EPI_STORE)
-            k = self._mm_epi(kx, att + "key.weight", EPI_STORE)
-            v = self._mm_epi(vx, att + "value.weight", EPI_STORE)
-            g = self._mm_epi(gx, att + "gate.weight", EPI_SILU)
+            r = self._mm_epi(rx, att + "receptance.weight", EPI_STORE, early=early)
+            k = self._mm_epi(kx, att + "key.weight", EPI_STORE, early=early)
+            v = self._mm_epi(vx, att + "value.weight", EPI_STORE, early=early)
+            g = self._mm_epi(gx, att + "gate.weight", EPI_SILU, early=early)
         y = torch.empty((T, D), dtype=torch.float32, device=dev)
         S_in = st2[1] if st2[1].is_contiguous() else st2[1].contiguous()
         S = torch.empty_like(S_in)                  # the caller's state stays as it is, as with the reference's copy
@@ -1036,7 +1040,7 @@ class RWKV:
                                      g.data_ptr(), out.data_ptr(), 64e-5, stream), "gn_gate")
         st2[0] = new_sx
         st2[1] = S
-        return self._mm_epi(out, att + "output.weight", EPI_RESIDUAL, aux=x, out=x)
+        return self._mm_epi(out, att + "output.weight", EPI_RESIDUAL, aux=x, out=x, early=early)
 
     def _tiled(self, name, t, reps):
         """A per-head / per-channel model vector repeated for `reps` sequences (cached: made once per batch size)."""
@@ -1046,7 +1050,7 @@ class RWKV:
             c = self._tile_cache[key] = t.reshape(-1).repeat(reps).contiguous()
         return c
 
-    def _ffn_seq(self, x, sx, i, rows=False):
+    def _ffn_seq(self, x, sx, i, rows=False, early=False):
         """ffn_seq / ffn_seq_v6 (model.py:995-1004, 1019-1029)."""
         w = self.w
         T = x.shape[0]
@@ -1061,12 +1065,12 @@ class RWKV:
             if rows:
                 r, vx = self._mm_fork([(rx, ffn + "receptance.weight", EPI_SIGMOID), (kx, ffn + "key.weight", EPI_RELU_SQ)])
             else:
-                r = self._mm_epi(rx, ffn + "receptance.weight", EPI_SIGMOID)
-                vx = self._mm_epi(kx, ffn + "key.weight", EPI_RELU_SQ)
+                r = self._mm_epi(rx, ffn + "receptance.weight", EPI_SIGMOID, early=early)
+                vx = self._mm_epi(kx, ffn + "key.weight", EPI_RELU_SQ, early=early)
             # x + r * (vx @ Wv), and the halving after every RESCALE_LAYER-th layer (model.py:1660-1662), in the store
             half = self.RESCALE_LAYER > 0 and (i + 1) % self.RESCALE_LAYER == 0
             return self._mm_epi(vx, ffn + "value.weight", EPI_MUL_RESIDUAL, aux=x, aux2=r, out_scale=0.5 if half else 1.0,
-                                out=x), new_sx
+                                out=x, early=early), new_sx
         r = torch.sigmoid(self._mm_seq(rx, ffn + "receptance.weight"))
         vx = torch.relu(self._mm_seq(kx, ffn + "key.weight")) ** 2
         out = r * self._mm_seq(vx, ffn + "value.weight")
@@ -1182,12 +1186,18 @@ class RWKV:
         self._seq_tok_ev[slot].record(torch.cuda.current_stream(self.device))
         return idx
 
-    def _forward_seq(self, tokens, state, full_output):
+    # The group norm of RWKV-5/6 divides by nearly nothing at the first positions of an empty state: there two correct
+    # summation orders of the same matmul end up percents apart, and the difference fades as 1 / T (state entries: 0.4 of
+    # their RMS after 100 tokens, 0.05 after 600).  Shorter prompts from an empty state keep the fp16 path's sums.
+    EARLY_PROMPT = 512
+
+    def _forward_seq(self, tokens, state, full_output, fresh=False):
         # (Replaying a prompt length that comes back as a CUDA graph was tried: with the copies of the state in and out
         # it was slower than these direct launches at 64, 256 and 1024 tokens.)
         w, a = self.w, self.args
         state = list(state)
         idx = self._stage_tokens(tokens)
+        early = fresh and self.version != 4 and len(tokens) < self.EARLY_PROMPT
         x = w["emb.weight"].index_select(0, idx)
         for i in range(a.n_layer):
             if self.version == 4:
@@ -1195,9 +1205,9 @@ class RWKV:
                 x, state[i * 5 + 4] = self._ffn_seq(x, state[i * 5 + 4], i)
             else:
                 st2 = [state[i * 3 + 0], state[i * 3 + 1]]
-                x = self._att_seq_v56(x, st2, i)
+                x = self._att_seq_v56(x, st2, i, early=early)
                 state[i * 3 + 0], state[i * 3 + 1] = st2
-                x, state[i * 3 + 2] = self._ffn_seq(x, state[i * 3 + 2], i)
+                x, state[i * 3 + 2] = self._ffn_seq(x, state[i * 3 + 2], i, early=early)
             if self._world > 1 and self.RESCALE_LAYER > 0 and (i + 1) % self.RESCALE_LAYER == 0:
                 x = x / 2           # (single GPU: fused into the ffn.value store)
         if not full_output:
@@ -1205,7 +1215,7 @@ class RWKV:
         xln = torch.empty_like(x)
         self._ln_mix(x.shape[0], x, None, w["ln_out.weight"], w["ln_out.bias"], 0, [], [], xx_out=xln)
         if full_output and self._world == 1:
-            out = self._mm_epi(xln, "head.weight", EPI_STORE)
+            out = self._mm_epi(xln, "head.weight", EPI_STORE, early=early)
         elif full_output or self._world > 1:
             out = self._mm_seq(xln, "head.weight")
             if not full_output:

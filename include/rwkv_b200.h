@@ -342,11 +342,13 @@ int rwkv_mm8_stream_take_error(uint32_t* sync_words, void* stream, int* error_ou
  * rwkv_mm8_seq_tc_take_error synchronises `stream` and returns/clears the workspace's error
  * word (1 if a bounded wait inside the tensor-core kernel gave up; outputs then undefined).
  * ------------------------------------------------------------------------------------- */
+enum { RWKV_SEQ_F16_SUMS = 0x100 };
 void rwkv_mm8_seq_set_path(int path);
 int rwkv_mm8_seq_tc_take_error(void* workspace, void* stream, int* error_out);
 size_t rwkv_mm8_seq_workspace_bytes(int64_t B, int64_t N, int64_t M);
 /* mm8_seq with a fused epilogue: RWKV_EPI_STORE, _SIGMOID, _RELU_SQ, _RESIDUAL (aux), _MUL_RESIDUAL (aux, aux2)
- * or _SILU applied to the fp32 sums with the roundings listed for rwkv_mm8_one_batch; aux, aux2: [B, M] in
+ * or _SILU applied to the fp32 sums with the roundings listed for rwkv_mm8_one_batch (RWKV_SEQ_F16_SUMS added to the
+ * epilogue: never the integer tensor-core kernel, the kernels and sums of the fp16 path); aux, aux2: [B, M] in
  * `dtype`, rows aux_stride / aux2_stride elements apart; y may alias aux.  What ffn_seq / cuda_att_seq apply
  * between matmuls (pkg/model.py:995-1004, 1346-1360). */
 int rwkv_mm8_seq_epi(int64_t B, int64_t N, int64_t M, const void* x, int64_t x_stride,
