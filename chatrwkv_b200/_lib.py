@@ -13,7 +13,7 @@ LIB_PATH = os.path.join(_HERE, "librwkv_b200.so")
 
 OK = 0
 F32, F16, BF16 = 0, 1, 2
-PRO_PLAIN, PRO_LN_MIX, PRO_WKV4 = 0, 1, 2
+PRO_PLAIN, PRO_LN_MIX, PRO_WKV4, PRO_GN_GATE = 0, 1, 2, 3
 ERR_UNSUPPORTED = -5
 MM8_WIDE_BUILD = 1
 SEQ_F16_SUMS = 0x100      # added to an epilogue of mm8_seq_epi
@@ -35,6 +35,23 @@ class Mm8Problem(C.Structure):
         ("k", C.c_void_p), ("v", C.c_void_p), ("t_decay", C.c_void_p), ("t_first", C.c_void_p),
         ("aa", C.c_void_p), ("bb", C.c_void_p), ("pp", C.c_void_p),
         ("aa_out", C.c_void_p), ("bb_out", C.c_void_p), ("pp_out", C.c_void_p),
+    ]
+
+
+class Mm8SeqProblem(C.Structure):
+    """rwkv_mm8_seq_problem, its prologue's fields in line."""
+    _fields_ = [
+        ("x", C.c_void_p), ("x_stride", C.c_int64), ("w", C.c_void_p), ("w_stride", C.c_int64),
+        ("mx", C.c_void_p), ("rx", C.c_void_p), ("my", C.c_void_p), ("ry", C.c_void_p),
+        ("y", C.c_void_p), ("y_stride", C.c_int64), ("M", C.c_int64),
+        ("epilogue", C.c_int32), ("out_scale", C.c_float),
+        ("aux", C.c_void_p), ("aux_stride", C.c_int64), ("aux2", C.c_void_p), ("aux2_stride", C.c_int64),
+        ("kind", C.c_int32), ("mode", C.c_int32),
+        ("sx", C.c_void_p), ("sx_stride", C.c_int64), ("ln_w", C.c_void_p), ("ln_b", C.c_void_p), ("mix", C.c_void_p),
+        ("xx_out", C.c_void_p), ("xx_stride", C.c_int64), ("new_state", C.c_void_p),
+        ("gate", C.c_void_p), ("gate_stride", C.c_int64), ("head", C.c_int32), ("eps", C.c_float),
+        ("k", C.c_void_p), ("v", C.c_void_p), ("t_decay", C.c_void_p), ("t_first", C.c_void_p),
+        ("aa", C.c_void_p), ("bb", C.c_void_p), ("pp", C.c_void_p),
     ]
 
 
@@ -95,6 +112,8 @@ SIGNATURES = {
     "rwkv_mm8_seq": (_i32, [_i64, _i64, _i64, _vp, _i64, _vp, _i64, _vp, _vp, _vp, _vp, _i32, _vp, _i64, _vp, _sz, _vp]),
     "rwkv_mm8_seq_epi": (_i32, [_i64, _i64, _i64, _vp, _i64, _vp, _i64, _vp, _vp, _vp, _vp, _i32, _vp, _i64, _i32, _vp, _i64, _vp, _i64,
                                 _f, _vp, _sz, _vp]),
+    "rwkv_mm8_seq_batch_workspace_bytes": (_sz, [C.POINTER(Mm8SeqProblem), _i32, _i64, _i64]),
+    "rwkv_mm8_seq_batch": (_i32, [C.POINTER(Mm8SeqProblem), _i32, _i64, _i64, _vp, _sz, _vp]),
     "rwkv_wkv4_workspace_bytes": (_sz, [_i64, _i64, _i64]),
     "rwkv_wkv4_seq": (_i32, [_i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _vp, _vp, _vp, _vp, _sz, _vp]),
     "rwkv_wkv4_forward": (_i32, [_i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _i32, _vp, _vp, _vp, _vp]),

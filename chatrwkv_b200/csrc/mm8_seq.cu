@@ -142,7 +142,7 @@ extern "C" int rwkv_mm8_seq_epi(int64_t B, int64_t N, int64_t M, const void* x, 
     const int erc = seq_epi_check(epi);
     if (erc != RWKV_OK) return erc;
     if (g_seq_path != 1 && !g_seq_single && !f16_sums && workspace != nullptr && dtype == RWKV_F16 && (B >= kI8MinRows || g_seq_path == 2)) {
-        const SeqI8Problem p = {x, x_stride, w, w_stride, mx, rx, my, ry, y, y_stride, M, epi};
+        const SeqI8Problem p = {x, x_stride, w, w_stride, mx, rx, my, ry, y, y_stride, M, epi, {}};
         const int rc = rwkv_mm8_seq_i8(1, &p, B, N, workspace, workspace_bytes, stream);
         if (rc != RWKV_ERR_UNSUPPORTED && rc != RWKV_ERR_WORKSPACE) return rc;   // else: the general kernels below
     }
@@ -171,4 +171,49 @@ extern "C" int rwkv_mm8_seq(int64_t B, int64_t N, int64_t M, const void* x, int6
                             void* y, int64_t y_stride, void* workspace, size_t workspace_bytes, void* stream) {
     return rwkv_mm8_seq_epi(B, N, M, x, x_stride, w, w_stride, mx, rx, my, ry, dtype, y, y_stride, RWKV_EPI_STORE, nullptr, 0,
                             nullptr, 0, 1.0f, workspace, workspace_bytes, stream);
+}
+
+extern "C" size_t rwkv_mm8_seq_batch_workspace_bytes(const rwkv_mm8_seq_problem* problems, int n, int64_t B, int64_t N) {
+    if (problems == nullptr || n < 1 || n > kSeqI8MaxProblems || B < 1 || N < 1) return 0;
+    int64_t M[kSeqI8MaxProblems];
+    for (int i = 0; i < n; ++i) {
+        if (problems[i].M < 1) return 0;
+        M[i] = problems[i].M;
+    }
+    return rwkv_mm8_seq_i8_workspace_bytes(n, B, N, M);
+}
+
+extern "C" int rwkv_mm8_seq_batch(const rwkv_mm8_seq_problem* problems, int n, int64_t B, int64_t N, void* workspace,
+                                  size_t workspace_bytes, void* stream) {
+    RWKV_CHECK_ARG(problems != nullptr && n >= 1 && n <= kSeqI8MaxProblems && B >= 1 && N >= 1 && B <= INT32_MAX && N <= INT32_MAX);
+    SeqI8Problem p[kSeqI8MaxProblems];
+    const rwkv_mm8_seq_prologue& q0 = problems[0].pro;
+    for (int i = 0; i < n; ++i) {
+        const rwkv_mm8_seq_problem& q = problems[i];
+        RWKV_CHECK_ARG(q.w && q.mx && q.rx && q.my && q.ry && q.y && q.x && q.M >= 1 && q.M <= INT32_MAX);
+        RWKV_CHECK_ARG(q.x_stride >= N && q.w_stride >= q.M && q.y_stride >= q.M);
+        RWKV_CHECK_ARG(q.pro.kind == q0.kind && q.pro.mode >= 0 && q.pro.mode <= 2);
+        if (q0.kind == RWKV_PRO_LN_MIX) RWKV_CHECK_ARG(q.pro.mode == 2 || (q.pro.mix != nullptr && q0.sx != nullptr));
+        p[i] = {q.x, q.x_stride, q.w, q.w_stride, q.mx, q.rx, q.my, q.ry, q.y, q.y_stride, q.M,
+                {q.epilogue, q.out_scale, q.aux, (long long)q.aux_stride, q.aux2, (long long)q.aux2_stride}, q.pro};
+        const int rc = seq_epi_check(p[i].epi);
+        if (rc != RWKV_OK) return rc;
+    }
+    switch (q0.kind) {
+    case RWKV_PRO_PLAIN: break;
+    case RWKV_PRO_LN_MIX:
+        RWKV_CHECK_ARG(q0.ln_w && q0.ln_b && (q0.sx_stride == 0 || q0.sx_stride >= N) && (q0.xx_out == nullptr || q0.xx_stride >= N));
+        break;
+    case RWKV_PRO_WKV4:
+        RWKV_CHECK_ARG(n == 1 && q0.k && q0.v && q0.t_decay && q0.t_first && q0.aa && q0.bb && q0.pp);
+        break;
+    case RWKV_PRO_GN_GATE:
+        RWKV_CHECK_ARG(n == 1 && q0.ln_w && q0.ln_b && q0.gate && q0.gate_stride >= N);
+        RWKV_CHECK_ARG((q0.head == 16 || q0.head == 32 || q0.head == 64 || q0.head == 128) && N % q0.head == 0);
+        break;
+    default: return RWKV_ERR_INVALID_ARG;
+    }
+    if (g_seq_path == 1 || g_seq_single) return RWKV_ERR_UNSUPPORTED;
+    if (q0.kind != RWKV_PRO_PLAIN && N > 16384) return RWKV_ERR_UNSUPPORTED;      // a row's channels in one block's registers
+    return rwkv_mm8_seq_i8(n, p, B, N, workspace, workspace_bytes, stream);
 }

@@ -172,7 +172,7 @@ __device__ __forceinline__ void tmem_ld8(int (&v)[8], uint32_t addr) {
 
 // ---- preparation: x' as digit planes, the row sums and scales ------------------------------------
 // One block per row (or per row and matrix); a thread owns a chunk of 16 k, kept in registers between the maximum and
-// the digits.
+// the digits.  What produces the row (LayerNorm + token shift, the one-step WKV, group norm + gate) runs in the same pass.
 __device__ __forceinline__ void load16(const __half* __restrict__ p, int k0, int N, bool vec, float (&out)[16]) {
     if (vec && k0 + 16 <= N) {
         const uint4 a = *reinterpret_cast<const uint4*>(p + k0), b = *reinterpret_cast<const uint4*>(p + k0 + 8);
@@ -185,7 +185,11 @@ __device__ __forceinline__ void load16(const __half* __restrict__ p, int k0, int
         for (int e = 0; e < 16; ++e) out[e] = (k0 + e < N) ? __half2float(p[k0 + e]) : 0.f;
     }
 }
-struct PrepProblem { const void* x; long long x_stride; const __half* ry; const __half* my; };
+struct PrepProblem {
+    rwkv_mm8_seq_prologue pro;                   // what makes the rows of x (RWKV_PRO_*)
+    const void* x; long long x_stride;
+    const __half* ry; const __half* my;
+};
 struct PrepArgs {
     PrepProblem p[kSeqI8MaxProblems];
     int nprob, T, N, nkb, TT, ntt, ntickets, vec;          // vec: every vector and row starts on a 16-byte boundary
@@ -226,15 +230,46 @@ __device__ __forceinline__ void block_reduce(float (&v)[NV], float (*sh)[32]) {
     }
 }
 
-// CH = 0: rows longer than 16384, read twice.
-template <int CH>
-__global__ void __launch_bounds__(1024) mm8_seq_i8_prep(const __grid_constant__ PrepArgs a) {
+__device__ __forceinline__ void load16f(const float* __restrict__ p, int k0, int N, bool vec, float (&out)[16]) {
+    if (vec && k0 + 16 <= N) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float4 v = *reinterpret_cast<const float4*>(p + k0 + 4 * i);
+            out[4 * i] = v.x; out[4 * i + 1] = v.y; out[4 * i + 2] = v.z; out[4 * i + 3] = v.w;
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) out[e] = (k0 + e < N) ? p[k0 + e] : 0.f;
+    }
+}
+template <typename F> __device__ __forceinline__ void store16(F* __restrict__ p, int k0, int N, bool vec, const float (&v)[16]) {
+    if (vec && k0 + 16 <= N) {
+        constexpr int PER = 16 / sizeof(F);
+#pragma unroll
+        for (int i = 0; i < 16 / PER; ++i) {
+            uint4 o;
+            F* h = reinterpret_cast<F*>(&o);
+#pragma unroll
+            for (int e = 0; e < PER; ++e) h[e] = from_f32<F>(v[i * PER + e]);
+            *reinterpret_cast<uint4*>(p + k0 + i * PER) = o;
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < 16; ++e)
+            if (k0 + e < N) p[k0 + e] = from_f32<F>(v[e]);
+    }
+}
+
+// PRO: where the rows of x come from (RWKV_PRO_*).  CH = 0 (RWKV_PRO_PLAIN only): rows longer than 16384, read twice.
+// MAXT: rows of up to 8192 run with 128 registers a thread (with 64 the LayerNorm form spills 500 bytes).
+template <int PRO, int CH, int MAXT>
+__global__ void __launch_bounds__(MAXT) mm8_seq_i8_prep(const __grid_constant__ PrepArgs a) {
     asm volatile("griddepcontrol.launch_dependents;");
     const int t = blockIdx.x, tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarp = nthr >> 5;
     __shared__ float sh[4][32];
     __shared__ long long shq[32];
     const bool vec = a.vec != 0;
-    const int N = a.N;
+    const int N = a.N, k0 = tid * 16;
     const int nchunk = a.nkb * (BKI / 16);
     const bool mine = tid < nchunk;
     float rv[16], mv[16];                                  // the first matrix's vectors do not depend on the work before
@@ -245,6 +280,94 @@ __global__ void __launch_bounds__(1024) mm8_seq_i8_prep(const __grid_constant__ 
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (t == 0 && blockIdx.y == 0)
         for (int i = tid; i < a.ntickets; i += nthr) a.tickets[i] = 0;
+
+    // ---- the row, common to all matrices of the launch
+    float xx[16] = {}, prev[16] = {};
+    if constexpr (PRO == RWKV_PRO_LN_MIX) {
+        // LayerNorm + token shift, rounding as rwkv_ln_mix; the previous row's output is the state or computed again
+        const rwkv_mm8_seq_prologue& q = a.p[0].pro;
+        const bool shift = q.sx != nullptr, own = !shift || t == 0 || q.sx_stride != 0;
+        const __half* x = static_cast<const __half*>(a.p[0].x) + (long long)t * a.p[0].x_stride;
+        load16(x, k0, N, vec, xx);
+        if (shift && own) load16(static_cast<const __half*>(q.sx) + (long long)t * q.sx_stride, k0, N, vec, prev);
+        else if (shift) load16(x - a.p[0].x_stride, k0, N, vec, prev);
+        float lw[16], lb[16];
+        load16(static_cast<const __half*>(q.ln_w), k0, N, vec, lw);
+        load16(static_cast<const __half*>(q.ln_b), k0, N, vec, lb);
+        float m[2] = {0.f, 0.f}, d[2] = {0.f, 0.f};
+#pragma unroll
+        for (int e = 0; e < 16; ++e) { m[0] += xx[e]; m[1] += prev[e]; }
+        block_reduce<2, false>(m, sh);
+        m[0] /= float(N); m[1] /= float(N);
+#pragma unroll
+        for (int e = 0; e < 16; ++e)
+            if (k0 + e < N) {
+                d[0] = fmaf(xx[e] - m[0], xx[e] - m[0], d[0]);
+                d[1] = fmaf(prev[e] - m[1], prev[e] - m[1], d[1]);
+            }
+        block_reduce<2, false>(d, sh);
+        const float r0 = rsqrtf(d[0] / float(N) + 1e-5f), r1 = rsqrtf(d[1] / float(N) + 1e-5f);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+            xx[e] = r16((xx[e] - m[0]) * r0 * lw[e] + lb[e]);
+            if (!own) prev[e] = r16((prev[e] - m[1]) * r1 * lw[e] + lb[e]);
+        }
+        if (blockIdx.y == 0) {
+            if (q.xx_out) store16(static_cast<__half*>(q.xx_out) + (long long)t * q.xx_stride, k0, N, vec, xx);
+            if (t == a.T - 1 && q.new_state) store16(static_cast<__half*>(q.new_state), k0, N, vec, xx);
+        }
+    } else if constexpr (PRO == RWKV_PRO_WKV4) {
+        // one step of the RWKV-4 recurrence per row, r * wkv with the roundings of rwkv_wkv4_seq; state in place
+        const rwkv_mm8_seq_prologue& q = a.p[0].pro;
+        const long long at = (long long)t * N;
+        float kk[16], vv[16], rr[16], w[16], u[16], aa[16], bb[16], pp[16];
+        load16(static_cast<const __half*>(q.k) + at, k0, N, vec, kk);
+        load16(static_cast<const __half*>(q.v) + at, k0, N, vec, vv);
+        load16(static_cast<const __half*>(a.p[0].x) + (long long)t * a.p[0].x_stride, k0, N, vec, rr);
+        load16f(q.t_decay, k0, N, vec, w);
+        load16f(q.t_first, k0, N, vec, u);
+        load16f(q.aa + at, k0, N, vec, aa);
+        load16f(q.bb + at, k0, N, vec, bb);
+        load16f(q.pp + at, k0, N, vec, pp);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+            float ww = u[e] + kk[e];
+            float p = fmaxf(pp[e], ww);
+            float e1 = expf(pp[e] - p), e2 = expf(ww - p);
+            const float y = (e1 * aa[e] + e2 * vv[e]) / (e1 * bb[e] + e2);
+            xx[e] = k0 + e < N ? r16(rr[e] * r16(y)) : 0.f;
+            ww = w[e] + pp[e];
+            p = fmaxf(ww, kk[e]);
+            e1 = expf(ww - p); e2 = expf(kk[e] - p);
+            aa[e] = e1 * aa[e] + e2 * vv[e];
+            bb[e] = e1 * bb[e] + e2;
+            pp[e] = p;
+        }
+        store16(q.aa + at, k0, N, vec, aa);
+        store16(q.bb + at, k0, N, vec, bb);
+        store16(q.pp + at, k0, N, vec, pp);
+    } else if constexpr (PRO == RWKV_PRO_GN_GATE) {
+        // group norm of each head (biased variance), ln_x in fp32, one rounding, times the gate: rwkv_v56_seq_gn_gate
+        const rwkv_mm8_seq_prologue& q = a.p[0].pro;
+        float y[16], lw[16], lb[16], g[16];
+        load16f(static_cast<const float*>(a.p[0].x) + (long long)t * a.p[0].x_stride, k0, N, vec, y);
+        load16f(static_cast<const float*>(q.ln_w), k0, N, vec, lw);
+        load16f(static_cast<const float*>(q.ln_b), k0, N, vec, lb);
+        load16(static_cast<const __half*>(q.gate) + (long long)t * q.gate_stride, k0, N, vec, g);
+        const int per = q.head / 16;                       // threads of a head: 1, 2, 4 or 8 neighbouring lanes
+        float s = 0.f, v = 0.f;
+#pragma unroll
+        for (int e = 0; e < 16; ++e) s += y[e];
+        for (int o = per >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        const float mean = s / float(q.head);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) v = fmaf(y[e] - mean, y[e] - mean, v);
+        for (int o = per >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        const float rstd = rsqrtf(v / float(q.head) + q.eps);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) xx[e] = k0 + e < N ? r16(r16((y[e] - mean) * rstd * lw[e] + lb[e]) * g[e]) : 0.f;
+    }
+
     // ---- digits, scale and sums for each matrix
     const int tt = t / a.TT, ti = t - tt * a.TT;
     const size_t plane = (size_t)a.TT * BKI;               // TT % 8 == 0: the three planes' rows share row % 8
@@ -255,7 +378,22 @@ __global__ void __launch_bounds__(1024) mm8_seq_i8_prep(const __grid_constant__ 
         float red[4] = {0.f, 0.f, 0.f, 0.f};               // maximum, SX, SXR, SXMY
         auto first = [&](int c) {
             float xv[16];
-            load16(x, c * 16, N, vec, xv);
+            if constexpr (PRO == RWKV_PRO_PLAIN) {
+                load16(x, c * 16, N, vec, xv);
+            } else if constexpr (PRO == RWKV_PRO_LN_MIX) {
+                float mix[16] = {};
+                if (p.pro.mode != 2) load16(static_cast<const __half*>(p.pro.mix), c * 16, N, vec, mix);
+#pragma unroll
+                for (int e = 0; e < 16; ++e) {
+                    const float o = p.pro.mode == 2 ? xx[e]
+                                    : p.pro.mode == 0 ? r16(r16(xx[e] * mix[e]) + r16(prev[e] * r16(1.0f - mix[e])))
+                                                      : r16(xx[e] + r16(r16(prev[e] - xx[e]) * mix[e]));
+                    xv[e] = c * 16 + e < N ? o : 0.f;
+                }
+            } else {
+#pragma unroll
+                for (int e = 0; e < 16; ++e) xv[e] = xx[e];
+            }
             if (CH == 0 || prob != (int)blockIdx.y) {
                 load16(p.ry, c * 16, N, vec, rv);
                 load16(p.my, c * 16, N, vec, mv);
@@ -732,6 +870,7 @@ int rwkv_mm8_seq_i8(int nprob, const SeqI8Problem* probs, int64_t T, int64_t N, 
     const int pc = p.pair ? 2 : 1;
     int tile = 0;
     bool vec = true;
+    const int pro = probs[0].pro.kind;
     auto al = [](const void* ptr, int64_t stride_bytes) { return reinterpret_cast<uintptr_t>(ptr) % 16 == 0 && stride_bytes % 16 == 0; };
     for (int i = 0; i < nprob; ++i) {
         const SeqI8Problem& q = probs[i];
@@ -748,10 +887,15 @@ int rwkv_mm8_seq_i8(int nprob, const SeqI8Problem* probs, int64_t T, int64_t N, 
         d.y = static_cast<__half*>(q.y); d.y_stride = q.y_stride; d.epi = q.epi; d.M = int(q.M); d.tile0 = tile;
         tile += int((q.M + BMC * pc - 1) / (BMC * pc)) * p.ntt;
         PrepProblem& r = pa.p[i];
-        r.x = q.x; r.x_stride = q.x_stride;
+        r.pro = q.pro; r.x = q.x; r.x_stride = q.x_stride;
         r.ry = static_cast<const __half*>(q.ry); r.my = static_cast<const __half*>(q.my);
-        vec = vec && al(q.x, q.x_stride * 2) && al(q.ry, 0) && al(q.my, 0);
+        const int xel = pro == RWKV_PRO_GN_GATE ? 4 : 2;
+        vec = vec && al(q.x, q.x_stride * xel) && al(q.ry, 0) && al(q.my, 0) && al(q.pro.sx, q.pro.sx_stride * 2) && al(q.pro.ln_w, 0) &&
+              al(q.pro.ln_b, 0) && al(q.pro.mix, 0) && al(q.pro.xx_out, q.pro.xx_stride * 2) && al(q.pro.new_state, 0) &&
+              al(q.pro.gate, q.pro.gate_stride * 2) && al(q.pro.k, 0) && al(q.pro.v, 0) && al(q.pro.t_decay, 0) && al(q.pro.t_first, 0) &&
+              al(q.pro.aa, 0) && al(q.pro.bb, 0) && al(q.pro.pp, 0);
     }
+    if (pro == RWKV_PRO_WKV4 && N % 8 != 0) vec = false;          // rows N apart
     pa.nprob = nprob; pa.vec = vec ? 1 : 0; pa.T = int(T); pa.N = int(N); pa.nkb = p.nkb; pa.TT = p.TT; pa.ntt = p.ntt;
     pa.ntickets = p.split > 1 ? p.parts / p.split * pc : 0;
     pa.images = ws + p.images; pa.consts = reinterpret_cast<RowConst*>(ws + p.consts); pa.tickets = reinterpret_cast<unsigned*>(ws + p.tickets);
@@ -783,10 +927,17 @@ int rwkv_mm8_seq_i8(int nprob, const SeqI8Problem* probs, int64_t T, int64_t N, 
     }
     const int nchunk = p.nkb * (BKI / 16);
     const int threads = std::min(1024, (nchunk + 31) / 32 * 32);
-    // few rows: a block per (row, matrix), so that they run side by side; many: a block per row
+    // few rows: a block per (row, matrix), so that they run side by side; many: the row is normalised once for all matrices
     const dim3 pgrid((unsigned)T, (unsigned)(T * nprob <= 2 * rwkv_sm_count() ? nprob : 1));
-    int rc = nchunk <= 1024 ? rwkv_launch_pdl(mm8_seq_i8_prep<1>, pgrid, dim3(threads), 0, st, pa)
-                            : rwkv_launch_pdl(mm8_seq_i8_prep<0>, pgrid, dim3(threads), 0, st, pa);
+    if (nchunk > 1024 && pro != RWKV_PRO_PLAIN) return RWKV_ERR_UNSUPPORTED;
+    auto prep = [&](auto kernel) { return rwkv_launch_pdl(kernel, pgrid, dim3(threads), 0, st, pa); };
+    const bool small = threads <= 512;
+    int rc;
+    if (nchunk > 1024) rc = prep(mm8_seq_i8_prep<RWKV_PRO_PLAIN, 0, 1024>);
+    else if (pro == RWKV_PRO_LN_MIX) rc = small ? prep(mm8_seq_i8_prep<RWKV_PRO_LN_MIX, 1, 512>) : prep(mm8_seq_i8_prep<RWKV_PRO_LN_MIX, 1, 1024>);
+    else if (pro == RWKV_PRO_WKV4) rc = small ? prep(mm8_seq_i8_prep<RWKV_PRO_WKV4, 1, 512>) : prep(mm8_seq_i8_prep<RWKV_PRO_WKV4, 1, 1024>);
+    else if (pro == RWKV_PRO_GN_GATE) rc = small ? prep(mm8_seq_i8_prep<RWKV_PRO_GN_GATE, 1, 512>) : prep(mm8_seq_i8_prep<RWKV_PRO_GN_GATE, 1, 1024>);
+    else rc = prep(mm8_seq_i8_prep<RWKV_PRO_PLAIN, 1, 1024>);
     if (rc != RWKV_OK) return rc;
     if (!p.pair) return rwkv_launch_pdl(mm8_seq_i8_kernel<1>, dim3(p.units), dim3(kThreadsI8), size_t(p.smem), st, a);
     return rwkv_launch_pdl_clustered(2, mm8_seq_i8_kernel<2>, dim3(p.units * 2), dim3(kThreadsI8), size_t(p.smem), st, a);

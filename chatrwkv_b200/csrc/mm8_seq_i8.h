@@ -9,6 +9,7 @@ struct SeqI8Problem {
     const void* mx; const void* rx; const void* my; const void* ry;
     void* y; int64_t y_stride; int64_t M;
     SeqEpi epi;
+    rwkv_mm8_seq_prologue pro;      // the same kind for all matrices of a launch
 };
 // Bytes for `rwkv_mm8_seq_i8` (0 where it does not apply); the first word of the workspace is its error word.
 size_t rwkv_mm8_seq_i8_workspace_bytes(int nprob, int64_t T, int64_t N, const int64_t* M);

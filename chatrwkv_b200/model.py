@@ -31,8 +31,8 @@ import torch
 import torch.nn.functional as F
 
 from . import _lib, ops, shard
-from ._lib import (EPI_MUL_RESIDUAL, EPI_RELU_SQ, EPI_RESIDUAL, EPI_SIGMOID, EPI_SILU, EPI_STORE, EPI_STORE_F32, check,
-                   lib)
+from ._lib import (EPI_MUL_RESIDUAL, EPI_RELU_SQ, EPI_RESIDUAL, EPI_SIGMOID, EPI_SILU, EPI_STORE, EPI_STORE_F32, PRO_GN_GATE,
+                   PRO_LN_MIX, PRO_PLAIN, PRO_WKV4, check, lib)
 
 STRATEGY_REGEX = r"^(?:(?:^|->) *(?:cuda(?::[\d]+)?|cpu|mps|dml) (?:fp(?:16|32)|bf16)(?:i8|i4|i3)?(?: \*[\d]+\+?)? *)+$"
 _MATRIX_KEYS = ("key.weight", "value.weight", "receptance.weight", "gate.weight", "output.weight", "head.weight")
@@ -349,6 +349,7 @@ class RWKV:
         self._stream = None
         self._mm = {}
         self._mm_pad = {}
+        self._seq_tables = {}
         self._fork_streams = []
         self._batch_fork = os.environ.get("RWKV_B200_BATCH_FORK", "1") != "0"
         self._v6_decay_fork = os.environ.get("RWKV_B200_V6_DECAY_FORK", "1") != "0"
@@ -889,37 +890,69 @@ class RWKV:
         y = out if out is not None else torch.empty((x.shape[0], M), dtype=torch.float16, device=x.device)
         return ops.mm8_seq_epi(x, wq, mx, rx, my, ry, y, epilogue, aux, aux2, out_scale)
 
-    def _mm_fork(self, jobs, extra=None):
-        """Independent matmuls of a batched decode step (r / k / v, or the two of the channel mix) on parallel
-        streams: `jobs` = [(x, name, epilogue)]; returns the outputs.  At a handful of rows every matmul is a
-        latency-bound chain of three short kernels, and the chains of independent matmuls overlap instead of queueing
-        (also inside a captured graph: the side streams fork from and join the capturing stream).  `extra`: one more
-        independent piece of work (a callable that launches on the current stream), run on a stream of its own."""
-        outs = [torch.empty((x.shape[0], self.w[name].shape[1]), dtype=torch.float16, device=x.device) for x, name, _ in jobs]
-        work = [lambda x=x, name=name, epi=epi, y=y: self._mm_epi(x, name, epi, out=y) for (x, name, epi), y in zip(jobs, outs)]
-        if extra is not None:
-            work.append(extra)
-        if not self._batch_fork or len(work) < 2:
-            for f in work:
-                f()
-            return outs
+    def _seq_group(self, kind, jobs, mode=0, ln=None, mixes=None):
+        """The table of a launch of 1..4 int8 matrices (rwkv_mm8_seq_batch) with what the model fixes, and its length:
+        `jobs` = [(name, epilogue)], `ln` = the names of the norm's weight and bias, `mixes` = names.  Made once; the
+        caller sets the activations' addresses.  (None, 0) when a matrix is kept in fp16 or split over ranks."""
+        key = jobs[0][0], kind
+        t = self._seq_tables.get(key)
+        if t is None:
+            w = self.w
+            if self._world > 1 or any(w[name].dtype != torch.uint8 for name, _ in jobs):
+                t = self._seq_tables[key] = (None, 0)
+                return t
+            arr = (_lib.Mm8SeqProblem * len(jobs))()
+            for i, (name, epi) in enumerate(jobs):
+                wq, mx, rx, my, ry = self._scales(name)
+                q = arr[i]
+                q.w, q.w_stride, q.M = wq.data_ptr(), wq.stride(0), wq.shape[1]
+                q.mx, q.rx, q.my, q.ry = mx.data_ptr(), rx.data_ptr(), my.data_ptr(), ry.data_ptr()
+                q.epilogue, q.out_scale, q.kind, q.mode = epi, 1.0, kind, mode
+                if ln is not None:
+                    q.ln_w, q.ln_b = w[ln[0]].data_ptr(), w[ln[1]].data_ptr()
+                if mixes is not None:
+                    q.mix = w[mixes[i]].data_ptr()
+            t = self._seq_tables[key] = (arr, len(jobs))
+        return t
+
+    def _ln_mix_group(self, x, sx, rows, jobs, mode, ln, mixes):
+        """LayerNorm, token shift and the matmuls of the mixes as two launches (operands, matmuls).  Returns the outputs and
+        the new shift state, or None where the separate launches have to run."""
+        T, D = x.shape
+        arr, n = self._seq_group(PRO_LN_MIX, jobs, mode, ln, mixes)
+        if arr is None:
+            return None
+        outs = [torch.empty((T, q.M), dtype=torch.float16, device=x.device) for q in arr]
+        new_sx = torch.empty_like(sx) if sx is not None else None
+        for q, y in zip(arr, outs):
+            q.x, q.x_stride, q.y, q.y_stride = x.data_ptr(), x.stride(0), y.data_ptr(), y.stride(0)
+        if sx is not None:
+            q = arr[0]
+            q.sx, q.sx_stride = sx.data_ptr(), (sx.stride(0) if rows else 0)
+            q.xx_out, q.xx_stride, q.new_state = (new_sx.data_ptr(), new_sx.stride(0), None) if rows else (None, 0, new_sx.data_ptr())
+        if not ops.mm8_seq_batch(arr, n, T, D, x.device):
+            return None
+        return outs, new_sx
+
+    def _fork(self, main_work, side_work):
+        """`side_work` on a stream of its own beside `main_work` (both callables that launch on the current stream), joined
+        before anything that follows; also inside a captured graph (the side stream forks from and joins the capturing one)."""
+        if not self._batch_fork:
+            side_work()
+            return main_work()
         main = torch.cuda.current_stream(self.device)
-        while len(self._fork_streams) < len(work) - 1:
+        if not self._fork_streams:
             self._fork_streams.append(torch.cuda.Stream(self.device))
-        start = torch.cuda.Event()
+        side = self._fork_streams[0]
+        start, done = torch.cuda.Event(), torch.cuda.Event()
         start.record(main)
-        joins = []
-        for side, f in zip(self._fork_streams, work[1:]):
-            side.wait_event(start)
-            with torch.cuda.stream(side):
-                f()
-                ev = torch.cuda.Event()
-                ev.record(side)
-                joins.append(ev)
-        work[0]()
-        for ev in joins:
-            main.wait_event(ev)
-        return outs
+        side.wait_event(start)
+        with torch.cuda.stream(side):
+            side_work()
+            done.record(side)
+        out = main_work()
+        main.wait_event(done)
+        return out
 
     def _att_seq_v4(self, x, st, i, rows=False):
         """cuda_att_seq (model.py:1346-1360): LayerNorm + mixes, r/k/v matmuls (sigmoid in the store), the WKV
@@ -927,18 +960,33 @@ class RWKV:
         w, a = self.w, self.args
         T, C = x.shape
         bb, att = f"blocks.{i}.", f"blocks.{i}.att."
-        kx, vx, rx = (torch.empty_like(x) for _ in range(3))
-        new_sx = torch.empty_like(st[i * 5 + 0])
-        self._ln_mix(T, x, st[i * 5 + 0], w[bb + "ln1.weight"], w[bb + "ln1.bias"], 0,
-                     [w[att + "time_mix_k"], w[att + "time_mix_v"], w[att + "time_mix_r"]], [kx, vx, rx],
-                     new_state=None if rows else new_sx, xx_out=new_sx if rows else None, rows=rows)
-        if self._world == 1 and rows:
-            r, k, v = self._mm_fork([(rx, att + "receptance.weight", EPI_SIGMOID), (kx, att + "key.weight", EPI_STORE),
-                                     (vx, att + "value.weight", EPI_STORE)])
-        elif self._world == 1:
-            r = self._mm_epi(rx, att + "receptance.weight", EPI_SIGMOID)
-            k = self._mm_epi(kx, att + "key.weight", EPI_STORE)             # fp16 k, v: the kernel widens them, as
-            v = self._mm_epi(vx, att + "value.weight", EPI_STORE)           # model.py:1355-1356 does before the op
+        done = self._ln_mix_group(x, st[i * 5 + 0], rows, [(att + "receptance.weight", EPI_SIGMOID), (att + "key.weight", EPI_STORE),
+                                                           (att + "value.weight", EPI_STORE)], 0, (bb + "ln1.weight", bb + "ln1.bias"),
+                                  [att + "time_mix_r", att + "time_mix_k", att + "time_mix_v"])
+        if done is not None:
+            (r, k, v), new_sx = done
+            arr, _ = self._seq_group(PRO_WKV4, [(att + "output.weight", EPI_RESIDUAL)]) if rows else (None, 0)
+            if arr is not None:     # T sequences of one step each: the recurrence runs in the launch that prepares the operand
+                aa, b_, pp = st[i * 5 + 1:i * 5 + 4]
+                ops._require(all(t.is_contiguous() for t in (aa, b_, pp)), "wkv needs contiguous tensors")
+                q = arr[0]
+                q.x, q.x_stride, q.k, q.v = r.data_ptr(), r.stride(0), k.data_ptr(), v.data_ptr()
+                q.t_decay, q.t_first = w[att + "time_decay"].data_ptr(), w[att + "time_first"].data_ptr()
+                q.aa, q.bb, q.pp = aa.data_ptr(), b_.data_ptr(), pp.data_ptr()
+                q.y, q.y_stride, q.aux, q.aux_stride = x.data_ptr(), x.stride(0), x.data_ptr(), x.stride(0)
+                if ops.mm8_seq_batch(arr, 1, T, r.shape[1], x.device):
+                    st[i * 5 + 0] = new_sx
+                    return x
+        else:
+            kx, vx, rx = (torch.empty_like(x) for _ in range(3))
+            new_sx = torch.empty_like(st[i * 5 + 0])
+            self._ln_mix(T, x, st[i * 5 + 0], w[bb + "ln1.weight"], w[bb + "ln1.bias"], 0,
+                         [w[att + "time_mix_k"], w[att + "time_mix_v"], w[att + "time_mix_r"]], [kx, vx, rx],
+                         new_state=None if rows else new_sx, xx_out=new_sx if rows else None, rows=rows)
+            if self._world == 1:
+                r = self._mm_epi(rx, att + "receptance.weight", EPI_SIGMOID)
+                k = self._mm_epi(kx, att + "key.weight", EPI_STORE)             # fp16 k, v: the kernel widens them, as
+                v = self._mm_epi(vx, att + "value.weight", EPI_STORE)           # model.py:1355-1356 does before the op
         if self._world == 1:
             if rows:        # T sequences of one step each: the operator's batch dimension, state [T, C]
                 ops.wkv4_seq(w[att + "time_decay"], w[att + "time_first"], k.view(T, 1, C), v.view(T, 1, C), k.view(T, 1, C),
@@ -1005,23 +1053,39 @@ class RWKV:
                 check(L.rwkv_tanh_regroup_f16(T, 1, h2.shape[1], h2.data_ptr(), h2.data_ptr(), s_), "tanh")
                 torch.ops.rwkv.gemm_fp16_cublas(h2, dw2, d2)
                 check(L.rwkv_v6_seq_decay(T, D, w[att + "time_decay"].data_ptr(), d2.data_ptr(), decay.data_ptr(), s_), "v6_seq_decay")
-            if not rows:
+            jobs = [(att + "receptance.weight", EPI_STORE), (att + "key.weight", EPI_STORE), (att + "value.weight", EPI_STORE),
+                    (att + "gate.weight", EPI_SILU)]
+
+            def matmuls():      # fp16-rounded r, k, v: the kernel widens them (model.py:1413, 1425-1427)
+                arr, n = self._seq_group(PRO_PLAIN, jobs)
+                if arr is not None and not early:
+                    outs = [torch.empty((T, q.M), dtype=torch.float16, device=dev) for q in arr]
+                    for q, xm, ym in zip(arr, (rx, kx, vx, gx), outs):
+                        q.x, q.x_stride, q.y, q.y_stride = xm.data_ptr(), xm.stride(0), ym.data_ptr(), ym.stride(0)
+                    if ops.mm8_seq_batch(arr, n, T, D, dev):
+                        return outs
+                return [self._mm_epi(xm, name, epi, early=early) for xm, (name, epi) in zip((rx, kx, vx, gx), jobs)]
+            if rows:
+                r, k, v, g = self._fork(matmuls, decay_chain)
+            else:
                 decay_chain()
+                r, k, v, g = matmuls()
         else:
-            kx, vx, rx, gx = (torch.empty_like(x) for _ in range(4))
-            self._ln_mix(T, x, st2[0], w[bb + "ln1.weight"], w[bb + "ln1.bias"], 0,
-                         [w[att + f"time_mix_{n}"] for n in "kvrg"], [kx, vx, rx, gx],
-                         new_state=None if rows else new_sx, xx_out=new_sx if rows else None, rows=rows)
             decay = w[att + "time_decay"].reshape(-1)
-        if rows:    # fp16-rounded r, k, v: the kernel widens them (model.py:1413, 1425-1427)
-            r, k, v, g = self._mm_fork([(rx, att + "receptance.weight", EPI_STORE), (kx, att + "key.weight", EPI_STORE),
-                                        (vx, att + "value.weight", EPI_STORE), (gx, att + "gate.weight", EPI_SILU)],
-                                       extra=decay_chain if self.version == 6 else None)
-        else:
-            r = self._mm_epi(rx, att + "receptance.weight", EPI_STORE, early=early)
-            k = self._mm_epi(kx, att + "key.weight", EPI_STORE, early=early)
-            v = self._mm_epi(vx, att + "value.weight", EPI_STORE, early=early)
-            g = self._mm_epi(gx, att + "gate.weight", EPI_SILU, early=early)
+            done = None if early else self._ln_mix_group(x, st2[0], rows, [(att + "receptance.weight", EPI_STORE), (att + "key.weight", EPI_STORE),
+                                                        (att + "value.weight", EPI_STORE), (att + "gate.weight", EPI_SILU)], 0,
+                                      (bb + "ln1.weight", bb + "ln1.bias"), [att + f"time_mix_{n}" for n in "rkvg"])
+            if done is not None:
+                (r, k, v, g), new_sx = done
+            else:
+                kx, vx, rx, gx = (torch.empty_like(x) for _ in range(4))
+                self._ln_mix(T, x, st2[0], w[bb + "ln1.weight"], w[bb + "ln1.bias"], 0,
+                             [w[att + f"time_mix_{n}"] for n in "kvrg"], [kx, vx, rx, gx],
+                             new_state=None if rows else new_sx, xx_out=new_sx if rows else None, rows=rows)
+                r = self._mm_epi(rx, att + "receptance.weight", EPI_STORE, early=early)
+                k = self._mm_epi(kx, att + "key.weight", EPI_STORE, early=early)
+                v = self._mm_epi(vx, att + "value.weight", EPI_STORE, early=early)
+                g = self._mm_epi(gx, att + "gate.weight", EPI_SILU, early=early)
         y = torch.empty((T, D), dtype=torch.float32, device=dev)
         S_in = st2[1] if st2[1].is_contiguous() else st2[1].contiguous()
         S = torch.empty_like(S_in)                  # the caller's state stays as it is, as with the reference's copy
@@ -1035,11 +1099,18 @@ class RWKV:
                           self.version != 6 else decay.view(1, T * D), u, y.view(1, T * D), model_layout=True, state_out=S)
         else:
             ops.wkv56_seq(self.version == 6, H, S_in, r, k, v, decay, u, y, model_layout=True, state_out=S)
+        st2[0] = new_sx
+        st2[1] = S
+        arr, _ = self._seq_group(PRO_GN_GATE, [(att + "output.weight", EPI_RESIDUAL)], ln=(att + "ln_x.weight", att + "ln_x.bias"))
+        if arr is not None and not early:
+            q = arr[0]
+            q.x, q.x_stride, q.gate, q.gate_stride, q.head, q.eps = y.data_ptr(), D, g.data_ptr(), g.stride(0), N, 64e-5
+            q.y, q.y_stride, q.aux, q.aux_stride = x.data_ptr(), x.stride(0), x.data_ptr(), x.stride(0)
+            if ops.mm8_seq_batch(arr, 1, T, D, dev):
+                return x
         out = h(T, D)
         check(L.rwkv_v56_seq_gn_gate(T, H, N, y.data_ptr(), w[att + "ln_x.weight"].data_ptr(), w[att + "ln_x.bias"].data_ptr(),
                                      g.data_ptr(), out.data_ptr(), 64e-5, stream), "gn_gate")
-        st2[0] = new_sx
-        st2[1] = S
         return self._mm_epi(out, att + "output.weight", EPI_RESIDUAL, aux=x, out=x, early=early)
 
     def _tiled(self, name, t, reps):
@@ -1055,20 +1126,23 @@ class RWKV:
         w = self.w
         T = x.shape[0]
         bb, ffn = f"blocks.{i}.", f"blocks.{i}.ffn."
-        kx, rx = torch.empty_like(x), torch.empty_like(x)
-        new_sx = torch.empty_like(sx)
         v6 = self.version == 6
-        self._ln_mix(T, x, sx, w[bb + "ln2.weight"], w[bb + "ln2.bias"], 1 if v6 else 0,
-                     [w[ffn + ("time_maa_k" if v6 else "time_mix_k")], w[ffn + ("time_maa_r" if v6 else "time_mix_r")]], [kx, rx],
-                     new_state=None if rows else new_sx, xx_out=new_sx if rows else None, rows=rows)
-        if self._world == 1:
-            if rows:
-                r, vx = self._mm_fork([(rx, ffn + "receptance.weight", EPI_SIGMOID), (kx, ffn + "key.weight", EPI_RELU_SQ)])
-            else:
+        half = self.RESCALE_LAYER > 0 and (i + 1) % self.RESCALE_LAYER == 0
+        mk, mr = (ffn + "time_maa_k", ffn + "time_maa_r") if v6 else (ffn + "time_mix_k", ffn + "time_mix_r")
+        done = None if early else self._ln_mix_group(x, sx, rows, [(ffn + "receptance.weight", EPI_SIGMOID), (ffn + "key.weight", EPI_RELU_SQ)],
+                                  1 if v6 else 0, (bb + "ln2.weight", bb + "ln2.bias"), [mr, mk])
+        if done is not None:
+            (r, vx), new_sx = done
+        else:
+            kx, rx = torch.empty_like(x), torch.empty_like(x)
+            new_sx = torch.empty_like(sx)
+            self._ln_mix(T, x, sx, w[bb + "ln2.weight"], w[bb + "ln2.bias"], 1 if v6 else 0, [w[mk], w[mr]], [kx, rx],
+                         new_state=None if rows else new_sx, xx_out=new_sx if rows else None, rows=rows)
+            if self._world == 1:
                 r = self._mm_epi(rx, ffn + "receptance.weight", EPI_SIGMOID, early=early)
                 vx = self._mm_epi(kx, ffn + "key.weight", EPI_RELU_SQ, early=early)
+        if self._world == 1:
             # x + r * (vx @ Wv), and the halving after every RESCALE_LAYER-th layer (model.py:1660-1662), in the store
-            half = self.RESCALE_LAYER > 0 and (i + 1) % self.RESCALE_LAYER == 0
             return self._mm_epi(vx, ffn + "value.weight", EPI_MUL_RESIDUAL, aux=x, aux2=r, out_scale=0.5 if half else 1.0,
                                 out=x, early=early), new_sx
         r = torch.sigmoid(self._mm_seq(rx, ffn + "receptance.weight"))
@@ -1161,9 +1235,17 @@ class RWKV:
                     x = self._att_seq_v56(x, st2, i, rows=True)
                     state[i * 3 + 0], state[i * 3 + 1] = st2
                     x, state[i * 3 + 2] = self._ffn_seq(x, state[i * 3 + 2], i, rows=True)
-            xln = torch.empty_like(x)
-            self._ln_mix(B, x, None, w["ln_out.weight"], w["ln_out.bias"], 0, [], [], xx_out=xln)
-            return self._mm_epi(xln, "head.weight", EPI_STORE).float(), state
+            return self._head_rows(x).float(), state
+
+    def _head_rows(self, x, early=False):
+        """ln_out and the head for every row of x: fp16 logits [T, V]."""
+        w = self.w
+        done = None if early else self._ln_mix_group(x, None, True, [("head.weight", EPI_STORE)], 2, ("ln_out.weight", "ln_out.bias"), None)
+        if done is not None:
+            return done[0][0]
+        xln = torch.empty_like(x)
+        self._ln_mix(x.shape[0], x, None, w["ln_out.weight"], w["ln_out.bias"], 0, [], [], xx_out=xln)
+        return self._mm_epi(xln, "head.weight", EPI_STORE, early=early)
 
     def _stage_tokens(self, tokens):
         """Token ids to the device through pinned memory (two slots, reused in turn): a copy from pageable memory would
@@ -1212,11 +1294,11 @@ class RWKV:
                 x = x / 2           # (single GPU: fused into the ffn.value store)
         if not full_output:
             x = x[-1:, :]
+        if full_output and self._world == 1:
+            return self._head_rows(x, early).float(), state
         xln = torch.empty_like(x)
         self._ln_mix(x.shape[0], x, None, w["ln_out.weight"], w["ln_out.bias"], 0, [], [], xx_out=xln)
-        if full_output and self._world == 1:
-            out = self._mm_epi(xln, "head.weight", EPI_STORE, early=early)
-        elif full_output or self._world > 1:
+        if full_output or self._world > 1:
             out = self._mm_seq(xln, "head.weight")
             if not full_output:
                 out = out[0]

@@ -162,6 +162,20 @@ def mm8_seq_epi(x, w, mx, rx, my, ry, y, epilogue, aux=None, aux2=None, out_scal
     return y
 
 
+def mm8_seq_batch(problems, n, B, N, device):
+    """1..4 matrices on B rows in one launch (`problems`: an array of `_lib.Mm8SeqProblem`; rwkv_mm8_seq_batch in the
+    header).  False where the tensor-core kernel does not take the operands: nothing has been launched then."""
+    nbytes = lib().rwkv_mm8_seq_batch_workspace_bytes(problems, n, B, N)
+    if nbytes == 0:
+        return False
+    ws = workspace(device, nbytes, "mm8_seq")
+    rc = lib().rwkv_mm8_seq_batch(problems, n, B, N, ws.data_ptr(), ws.numel(), _stream(device))
+    if rc == _lib.ERR_UNSUPPORTED:
+        return False
+    check(rc, "mm8_seq_batch")
+    return True
+
+
 def wkv4_seq(w, u, k, v, y, aa, bb, pp, r=None):
     """WKV-v4 over k, v [T, C] (or [B, T, C]) with the state aa, bb, pp updated in place, parallel in time from 33
     steps on; with `r`, y = r * wkv rounded as cuda_att_seq does (rwkv_wkv4_seq in the header)."""

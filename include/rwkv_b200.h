@@ -154,7 +154,7 @@ enum {
  *                    WKV (pkg/model.py:1044-1055) on k, v, t_decay, t_first and the state
  *                    aa, bb, pp, uses r*wkv, and stores the new state to aa_out, bb_out,
  *                    pp_out, which must not alias aa, bb, pp. */
-enum { RWKV_PRO_PLAIN = 0, RWKV_PRO_LN_MIX = 1, RWKV_PRO_WKV4 = 2 };
+enum { RWKV_PRO_PLAIN = 0, RWKV_PRO_LN_MIX = 1, RWKV_PRO_WKV4 = 2, RWKV_PRO_GN_GATE = 3 /* rwkv_mm8_seq_batch */ };
 
 typedef struct rwkv_mm8_problem {
     const void* x;          /* [N] activations (see the prologues) */
@@ -361,6 +361,46 @@ int rwkv_mm8_seq(int64_t B, int64_t N, int64_t M, const void* x, int64_t x_strid
                  const uint8_t* w, int64_t w_stride,
                  const void* mx, const void* rx, const void* my, const void* ry, int dtype,
                  void* y, int64_t y_stride, void* workspace, size_t workspace_bytes, void* stream);
+
+/* 1..4 matrices of N in-features applied to B rows in one launch (fp16), with what precedes the matmuls in the sequence
+ * functions computed in the same pass that prepares the operands.  All problems of a call share `pro.kind`:
+ *   RWKV_PRO_PLAIN    x [B, N] as given, each problem its own.
+ *   RWKV_PRO_LN_MIX   x is the residual stream (the first problem's counts, as do ln_w, ln_b [N], sx, xx_out, new_state):
+ *                     LayerNorm, then per problem the token-shift `mix` [N] (rwkv_ln_mix: mode 0 RWKV-4/5, mode 1 RWKV-6;
+ *                     mode 2: the LayerNorm alone).  sx_stride == 0: the rows are consecutive tokens, sx [N] the state before the
+ *                     first; else row t is a sequence of its own with its state at sx + t * sx_stride.  xx_out (may be
+ *                     NULL): the LayerNorm output of every row; new_state (may be NULL): that of the last row.
+ *   RWKV_PRO_WKV4     one problem: x = r [B, N], one step of the RWKV-4 recurrence per row on the states aa, bb, pp [B, N]
+ *                     (updated in place), k, v [B, N] fp16; the matmul's row is r * wkv (rwkv_wkv4_seq with T = 1).
+ *   RWKV_PRO_GN_GATE  one problem: x [B, N] in fp32, group norm over each `head` channels with eps and ln_w, ln_b in
+ *                     fp32, times `gate` fp16 (rwkv_v56_seq_gn_gate).  head: 16, 32, 64 or 128.
+ * Everything else as rwkv_mm8_seq_epi.  RWKV_ERR_UNSUPPORTED where the tensor-core kernel does not take the operands
+ * (w not 16-byte aligned, N > 65536, or more than 16384 with a prologue; CUDA cores forced): the caller then makes the
+ * separate calls.  `workspace` as for rwkv_mm8_seq (the first word is its error word). */
+typedef struct {
+    int32_t kind, mode;
+    const void* sx; int64_t sx_stride;
+    const void* ln_w; const void* ln_b; const void* mix;
+    void* xx_out; int64_t xx_stride; void* new_state;
+    const void* gate; int64_t gate_stride;
+    int32_t head; float eps;
+    const void* k; const void* v;
+    const float* t_decay; const float* t_first;
+    float* aa; float* bb; float* pp;
+} rwkv_mm8_seq_prologue;
+typedef struct {
+    const void* x; int64_t x_stride;
+    const uint8_t* w; int64_t w_stride;
+    const void* mx; const void* rx; const void* my; const void* ry;
+    void* y; int64_t y_stride; int64_t M;
+    int32_t epilogue; float out_scale;
+    const void* aux; int64_t aux_stride;
+    const void* aux2; int64_t aux2_stride;
+    rwkv_mm8_seq_prologue pro;
+} rwkv_mm8_seq_problem;
+size_t rwkv_mm8_seq_batch_workspace_bytes(const rwkv_mm8_seq_problem* problems, int n, int64_t B, int64_t N);
+int rwkv_mm8_seq_batch(const rwkv_mm8_seq_problem* problems, int n, int64_t B, int64_t N, void* workspace,
+                       size_t workspace_bytes, void* stream);
 
 /* ---------------------------------------------------------------------------------------
  * WKV-v4 — replaces cuda_wkv_forward<F> (pkg/cuda/operators.cu:11-58) behind
