@@ -11,7 +11,10 @@
 // probability for top-k comes from the same search with counts instead of sums.  A round costs one cluster
 // barrier: every CTA pushes its fifteen partial sums into every CTA's shared memory (remote stores), and every
 // CTA adds the eight partials in rank order, so all CTAs take the same decisions.  Sums are taken in a fixed
-// order: the same inputs give the same token.
+// order: the same inputs give the same token.  What bounds a call is the chain of cluster barriers (1-1.5 us each) and
+// the sums between them: 62 us per draw at 65536 ids with sixteen barriers, fifteen 5-shuffle sums per round and every
+// thread adding all fifteen totals; 41 us with the sums folded across lanes, one total per lane, no barriers for the
+// largest probability and the total, and the search ended once a single id is left in the bracket.
 //
 // Differences from the reference that cannot be avoided: its cumulative sum runs in sorted order and ours in id
 // order, so a cutoff that hinges on the last ulp of a sum may fall one value higher or lower; ties at the top-k
@@ -116,17 +119,54 @@ __device__ __forceinline__ float cluster_max(SampleShared& sh, unsigned rank, in
     return s;
 }
 
+// Sixteen sums per thread over the cluster; lane i (< 16) of every warp of every CTA gets sum i.  The warp part is the
+// butterfly of warp_sum with half of the values dropped at each step (16 shuffles instead of 80, the same pairs added in
+// the same order), the rest is added in warp and rank order.
+__device__ __forceinline__ float cluster_sum16(SampleShared& sh, unsigned rank, int& parity, float (&v)[16]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int n = 8; n >= 1; n >>= 1) {
+        const bool upper = (lane & (2 * n)) != 0;
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+            const float mine = upper ? v[i + n] : v[i], other = upper ? v[i] : v[i + n];
+            v[i] = mine + __shfl_xor_sync(0xffffffffu, other, 2 * n);
+        }
+    }
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);           // lanes 2i and 2i + 1 hold sum i
+    if ((lane & 1) == 0) sh.warp_part[warp][lane >> 1] = v[0];
+    __syncthreads();
+    if (threadIdx.x < 16 * kSampleCtas) {
+        const int i = threadIdx.x & 15, d = threadIdx.x >> 4;
+        float s = 0.f;
+#pragma unroll
+        for (int q = 0; q < kSampleWarps; ++q) s += sh.warp_part[q][i];
+        push_f32(&sh.slot[parity][rank][i], unsigned(d), s);
+    }
+    cluster_barrier();
+    float s = 0.f;
+#pragma unroll
+    for (int q = 0; q < kSampleCtas; ++q) s += sh.slot[parity][q][lane & 15];
+    parity ^= 1;
+    return s;
+}
+
 // Largest bit pattern v (as a non-negative float) with  sum{ w_i : p_i >= v } >= target,  w_i = p_i (COUNT = false)
-// or 1 (COUNT = true); 0 if even v = 0 fails.  Eight rounds of four bits.
+// or 1 (COUNT = true); 0 if even v = 0 fails.  Eight rounds of four bits.  For sums the search ends once the bracket
+// [v, v + 2^shift) holds a single probability: any cutoff inside it keeps the same ids (a trained model's 65536 logits end
+// after five or six rounds).  `total`: the sum of all p_i, taken along in the first round.
 template <bool COUNT>
 __device__ __forceinline__ float search_threshold(SampleShared& sh, unsigned rank, int& parity, const float (&p)[kSamplePer],
-                                                  const bool (&valid)[kSamplePer], float target) {
+                                                  const bool (&valid)[kSamplePer], float target, float all, float& total) {
     uint32_t v = 0;
+    float above = 0.f;                                       // sum{ p_i : p_i >= v + 16 << shift }: what lies over the bracket
+    const int lane = threadIdx.x & 31;
 #pragma unroll 1
     for (int shift = 28; shift >= 0; shift -= 4) {
-        float part[kFan], tot[kFan];
+        float part[16];
 #pragma unroll
         for (int j = 0; j < kFan; ++j) part[j] = 0.f;
+        part[kFan] = all;
 #pragma unroll
         for (int i = 0; i < kSamplePer; ++i) {
             if (valid[i]) {
@@ -137,13 +177,19 @@ __device__ __forceinline__ float search_threshold(SampleShared& sh, unsigned ran
                     if (bits >= (v | (uint32_t(j + 1) << shift))) part[j] += w;
             }
         }
-        cluster_sum<kFan>(sh, rank, parity, part, tot);
-        int best = 0;
-#pragma unroll
-        for (int j = 0; j < kFan; ++j)
-            if (tot[j] >= target) best = j + 1;         // the sums fall as j rises: the last that holds
+        const float tot = cluster_sum16(sh, rank, parity, part);
+        if (shift == 28) total = __shfl_sync(0xffffffffu, tot, kFan);
+        // the sums fall as j rises: the last that holds
+        const uint32_t holds = __ballot_sync(0xffffffffu, lane < kFan && tot >= target);
+        int best = 32 - __clz(holds);
         if (shift == 28 && best > 7) best = 7;          // bit 31 is the sign
         v |= uint32_t(best) << shift;
+        if (!COUNT) {
+            if (best < kFan) above = __shfl_sync(0xffffffffu, tot, best);
+            const float in = best > 0 ? __shfl_sync(0xffffffffu, tot, best - 1) - above : INFINITY;
+            const float fv = __uint_as_float(v);
+            if (best > 0 && fv > 1e-5f && in < 1.5f * fv) break;      // the sums carry ~1e-7: one probability, not two
+        }
     }
     return __uint_as_float(v);
 }
@@ -186,33 +232,33 @@ __global__ void __cluster_dims__(kSampleCtas, 1, 1) __launch_bounds__(kSampleThr
     }
     cluster_sum<1>(sh, rank, parity, one, tot1);
     const float inv_z = 1.0f / tot1[0];
-    float pmax = 0.f;
-    one[0] = 0.f;
+    const float pmax = inv_z;                           // the likeliest id's expf(0) * inv_z
+    float all = 0.f;
 #pragma unroll
     for (int i = 0; i < kSamplePer; ++i) {
         p[i] *= inv_z;
-        one[0] += p[i];
-        pmax = fmaxf(pmax, p[i]);
+        all += p[i];
     }
-    cluster_sum<1>(sh, rank, parity, one, tot1);
-    const float total = tot1[0];
-    pmax = cluster_max(sh, rank, parity, pmax);
 
     // temperature 0 means greedy: temperature 1, top_p 0 (utils.py:56-58)
     float temperature = a.temperature, top_p = a.top_p;
     if (temperature == 0.f) { temperature = 1.f; top_p = 0.f; }
 
     // nucleus cutoff (utils.py:64-68): probabilities below it are dropped
-    float cutoff;
-    if (top_p <= 0.f || !(total >= top_p)) cutoff = pmax;
-    else cutoff = search_threshold<false>(sh, rank, parity, p, valid, top_p);
+    float cutoff = pmax;
+    if (top_p > 0.f) {
+        float total = 0.f;
+        const float found = search_threshold<false>(sh, rank, parity, p, valid, top_p, all, total);
+        if (total >= top_p) cutoff = found;
+    }
 
     // top-k (utils.py:69-70): everything but the k most likely is dropped; ties at the boundary by lowest id
     float kth = 0.f;
     int ties_kept = 0x7fffffff;
     const bool use_k = a.top_k > 0 && a.top_k < a.V;
     if (use_k) {
-        kth = search_threshold<true>(sh, rank, parity, p, valid, float(a.top_k));
+        float ignored;
+        kth = search_threshold<true>(sh, rank, parity, p, valid, float(a.top_k), 0.f, ignored);
         float gt[1] = {0.f}, gtt[1];
 #pragma unroll
         for (int i = 0; i < kSamplePer; ++i) gt[0] += (valid[i] && p[i] > kth) ? 1.f : 0.f;
