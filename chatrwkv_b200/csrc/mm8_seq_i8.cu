@@ -114,6 +114,20 @@ template <int PAIR> __device__ __forceinline__ void tma_load_2d(uint32_t dst, co
         asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                      ::"r"(dst), "l"((uint64_t)map), "r"(x), "r"(y), "r"(bar) : "memory");
 }
+// the same with an L2 eviction policy
+template <int PAIR> __device__ __forceinline__ void tma_load_2d_hint(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar, uint64_t policy) {
+    if constexpr (PAIR == 2)
+        asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;"
+                     ::"r"(dst), "l"((uint64_t)map), "r"(x), "r"(y), "r"(bar), "l"(policy) : "memory");
+    else
+        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;"
+                     ::"r"(dst), "l"((uint64_t)map), "r"(x), "r"(y), "r"(bar), "l"(policy) : "memory");
+}
+__device__ __forceinline__ uint64_t evict_first_policy() {
+    uint64_t p;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
 // Shared-memory matrix descriptor, 128-byte swizzle.  Both operands are stored as rows of 128 bytes whose 16-byte
 // chunks are permuted by (row % 8): for W a row is one k and its bytes are columns (MN-major), for the token planes a
 // row is one token and its bytes are k (K-major); 8-row groups follow each other at 1024 bytes.
@@ -672,6 +686,10 @@ __global__ void __launch_bounds__(kThreadsI8, 1) mm8_seq_i8_kernel(const __grid_
             uint32_t ph = 1;                                           // the stages start empty
             const uint32_t smem0 = su(smem);
             const int xrows = 3 * a.TT;                                // rows of one K block of the token planes
+            // With one token tile every byte of W is read once: it leaves L2 first, so that the activations, the norms' and
+            // scale vectors and the code of the next layers are still there (a 7B layer streams 1.6 times the L2).
+            const bool once = a.ntt == 1;
+            const uint64_t policy = evict_first_policy();
             auto full_of = [&](int st) { return PAIR == 2 ? in_cta(full0 + st * 8, 0) : full0 + st * 8; };
             Item tl;
             for (int seg = 0; ok && item_of<PAIR>(a, unit, seg, tl); ++seg) {
@@ -681,7 +699,8 @@ __global__ void __launch_bounds__(kThreadsI8, 1) mm8_seq_i8_kernel(const __grid_
                 auto load_w = [&](int i, int st) {
                     if (elect_one()) {
                         if (crank == 0) bar_expect(full0 + st * 8, PAIR * stage_bytes);
-                        tma_load_2d<PAIR>(smem0 + st * stage_bytes, map, n0, (tl.kb0 + i) * BKI, full_of(st));
+                        if (once) tma_load_2d_hint<PAIR>(smem0 + st * stage_bytes, map, n0, (tl.kb0 + i) * BKI, full_of(st), policy);
+                        else tma_load_2d<PAIR>(smem0 + st * stage_bytes, map, n0, (tl.kb0 + i) * BKI, full_of(st));
                     }
                 };
                 auto load_x = [&](int st) {
