@@ -185,18 +185,81 @@ __device__ __forceinline__ void tmem_ld8(int (&v)[8], uint32_t addr) {
 }
 
 // ---- preparation: x' as digit planes, the row sums and scales ------------------------------------
-// One block per row (or per row and matrix); a thread owns a chunk of 16 k, kept in registers between the maximum and
-// the digits.  What produces the row (LayerNorm + token shift, the one-step WKV, group norm + gate) runs in the same pass.
-__device__ __forceinline__ void load16(const __half* __restrict__ p, int k0, int N, bool vec, float (&out)[16]) {
-    if (vec && k0 + 16 <= N) {
-        const uint4 a = *reinterpret_cast<const uint4*>(p + k0), b = *reinterpret_cast<const uint4*>(p + k0 + 8);
-        const __half* ah = reinterpret_cast<const __half*>(&a);
-        const __half* bh = reinterpret_cast<const __half*>(&b);
+// One block per row (or per row and matrix); a thread owns E neighbouring k.  What produces the row (LayerNorm + token
+// shift, the one-step WKV, group norm + gate) runs in the same pass.  A block is a chain of latencies: one trip to memory,
+// two to four reductions, and the code itself, which the streamed weights have evicted (with 16 k a thread a launch of 16
+// rows took 10 us after its wait, 2.5 us when repeated alone).  So few rows run with E = 4: short code, and the weights'
+// vectors fetched before the dependency wait.  With many rows what counts is how many blocks an SM holds: E = 16, rows
+// kept as fp16, the vectors read when needed.
+template <int E> struct HV {                     // E fp16 values
+    __half2 h[E / 2];
+    __device__ __forceinline__ float operator[](int e) const { return (e & 1) ? __high2float(h[e >> 1]) : __low2float(h[e >> 1]); }
+    __device__ __forceinline__ void set(int e, float v) {
+        const __half x = __float2half_rn(v);
+        h[e >> 1] = (e & 1) ? __halves2half2(__low2half(h[e >> 1]), x) : __halves2half2(x, __high2half(h[e >> 1]));
+    }
+};
+template <int BYTES> struct VecOf { typedef uint4 T; };
+template <> struct VecOf<8> { typedef uint2 T; };
+template <> struct VecOf<4> { typedef uint32_t T; };
+template <int E> __device__ __forceinline__ HV<E> zero_hv() {
+    HV<E> o;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) { out[e] = __half2float(ah[e]); out[8 + e] = __half2float(bh[e]); }
+    for (int i = 0; i < E / 2; ++i) o.h[i] = __float2half2_rn(0.f);
+    return o;
+}
+template <int E, bool CONSTANT = false>          // CONSTANT: never written while kernels run (weights)
+__device__ __forceinline__ HV<E> load_hv(const void* ptr, long long k0, int N, bool vec) {
+    const __half* p = static_cast<const __half*>(ptr);
+    HV<E> o = zero_hv<E>();
+    if (vec && k0 + E <= N) {
+        typedef typename VecOf<E * 2>::T V;
+        const V* q = reinterpret_cast<const V*>(p + k0);
+        V v[E * 2 / sizeof(V)];
+#pragma unroll
+        for (int i = 0; i < int(E * 2 / sizeof(V)); ++i) v[i] = CONSTANT ? __ldg(q + i) : q[i];
+        memcpy(&o, v, sizeof(o));
     } else {
 #pragma unroll
-        for (int e = 0; e < 16; ++e) out[e] = (k0 + e < N) ? __half2float(p[k0 + e]) : 0.f;
+        for (int e = 0; e < E; ++e)
+            if (k0 + e < N) o.set(e, __half2float(p[k0 + e]));
+    }
+    return o;
+}
+template <int E> __device__ __forceinline__ void store_hv(void* ptr, int k0, int N, bool vec, const HV<E>& v) {
+    __half* p = static_cast<__half*>(ptr);
+    if (vec && k0 + E <= N) {
+        typedef typename VecOf<E * 2>::T V;
+        V o[E * 2 / sizeof(V)];
+        memcpy(o, &v, sizeof(o));
+#pragma unroll
+        for (int i = 0; i < int(E * 2 / sizeof(V)); ++i) reinterpret_cast<V*>(p + k0)[i] = o[i];
+    } else {
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+            if (k0 + e < N) p[k0 + e] = __float2half_rn(v[e]);
+    }
+}
+template <int E> __device__ __forceinline__ void load_f(const float* __restrict__ p, int k0, int N, bool vec, float (&out)[E]) {
+    if (vec && k0 + E <= N) {
+#pragma unroll
+        for (int i = 0; i < E / 4; ++i) {
+            const float4 v = reinterpret_cast<const float4*>(p + k0)[i];
+            out[4 * i] = v.x; out[4 * i + 1] = v.y; out[4 * i + 2] = v.z; out[4 * i + 3] = v.w;
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < E; ++e) out[e] = (k0 + e < N) ? p[k0 + e] : 0.f;
+    }
+}
+template <int E> __device__ __forceinline__ void store_f(float* p, int k0, int N, bool vec, const float (&v)[E]) {
+    if (vec && k0 + E <= N) {
+#pragma unroll
+        for (int i = 0; i < E / 4; ++i) reinterpret_cast<float4*>(p + k0)[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+    } else {
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+            if (k0 + e < N) p[k0 + e] = v[e];
     }
 }
 struct PrepProblem {
@@ -209,21 +272,6 @@ struct PrepArgs {
     int nprob, T, N, nkb, TT, ntt, ntickets, vec;          // vec: every vector and row starts on a 16-byte boundary
     uint8_t* images; RowConst* consts; unsigned* tickets;
 };
-__device__ __forceinline__ void store_digits(const float (&xp)[16], float up, uint8_t* dst, size_t plane_bytes, int& isum) {
-    uint32_t d[3][4] = {};
-#pragma unroll
-    for (int e = 0; e < 16; ++e) {
-        const int q = __float2int_rn(xp[e] * up);
-        isum += q;
-        const int d0 = (int)(int8_t)(q & 255), q1 = (q - d0) >> 8;
-        const int d1 = (int)(int8_t)(q1 & 255), d2 = (q1 - d1) >> 8;
-        d[0][e >> 2] |= (uint32_t)(d0 & 255) << (8 * (e & 3));
-        d[1][e >> 2] |= (uint32_t)(d1 & 255) << (8 * (e & 3));
-        d[2][e >> 2] |= (uint32_t)(d2 & 255) << (8 * (e & 3));
-    }
-#pragma unroll
-    for (int i = 0; i < 3; ++i) *reinterpret_cast<uint4*>(dst + i * plane_bytes) = make_uint4(d[i][0], d[i][1], d[i][2], d[i][3]);
-}
 // Sums (MAX0: the first value's maximum) of NV values per thread over the block; every thread gets the results.
 template <int NV, bool MAX0>
 __device__ __forceinline__ void block_reduce(float (&v)[NV], float (*sh)[32]) {
@@ -238,83 +286,60 @@ __device__ __forceinline__ void block_reduce(float (&v)[NV], float (*sh)[32]) {
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-        float t = sh[i][0];
-        for (int w = 1; w < nwarp; ++w) t = (MAX0 && i == 0) ? fmaxf(t, sh[i][w]) : t + sh[i][w];
-        v[i] = t;
+        const float t = lane < nwarp ? sh[i][lane] : 0.f;      // (maxima are of magnitudes)
+        v[i] = (MAX0 && i == 0) ? warp_max(t) : warp_sum(t);
     }
 }
 
-__device__ __forceinline__ void load16f(const float* __restrict__ p, int k0, int N, bool vec, float (&out)[16]) {
-    if (vec && k0 + 16 <= N) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float4 v = *reinterpret_cast<const float4*>(p + k0 + 4 * i);
-            out[4 * i] = v.x; out[4 * i + 1] = v.y; out[4 * i + 2] = v.z; out[4 * i + 3] = v.w;
-        }
-    } else {
-#pragma unroll
-        for (int e = 0; e < 16; ++e) out[e] = (k0 + e < N) ? p[k0 + e] : 0.f;
-    }
-}
-template <typename F> __device__ __forceinline__ void store16(F* __restrict__ p, int k0, int N, bool vec, const float (&v)[16]) {
-    if (vec && k0 + 16 <= N) {
-        constexpr int PER = 16 / sizeof(F);
-#pragma unroll
-        for (int i = 0; i < 16 / PER; ++i) {
-            uint4 o;
-            F* h = reinterpret_cast<F*>(&o);
-#pragma unroll
-            for (int e = 0; e < PER; ++e) h[e] = from_f32<F>(v[i * PER + e]);
-            *reinterpret_cast<uint4*>(p + k0 + i * PER) = o;
-        }
-    } else {
-#pragma unroll
-        for (int e = 0; e < 16; ++e)
-            if (k0 + e < N) p[k0 + e] = from_f32<F>(v[e]);
-    }
-}
-
-// PRO: where the rows of x come from (RWKV_PRO_*).  CH = 0 (RWKV_PRO_PLAIN only): rows longer than 16384, read twice.
-// MAXT: rows of up to 8192 run with 128 registers a thread (with 64 the LayerNorm form spills 500 bytes).
-template <int PRO, int CH, int MAXT>
-__global__ void __launch_bounds__(MAXT) mm8_seq_i8_prep(const __grid_constant__ PrepArgs a) {
+// PRO: where the rows of x come from (RWKV_PRO_*).  LOOP (RWKV_PRO_PLAIN only): a thread owns every blockDim-th E k and
+// reads the row twice (the second time from L1); else one chunk per thread.  PRE: the vectors of the first matrix and of
+// the prologue are fetched ahead of the dependency wait.
+template <int PRO, int E, bool LOOP, bool PRE, int MAXT, int MINB>
+__global__ void __launch_bounds__(MAXT, MINB) mm8_seq_i8_prep(const __grid_constant__ PrepArgs a) {
     asm volatile("griddepcontrol.launch_dependents;");
     const int t = blockIdx.x, tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarp = nthr >> 5;
     __shared__ float sh[4][32];
     __shared__ long long shq[32];
     const bool vec = a.vec != 0;
-    const int N = a.N, k0 = tid * 16;
-    const int nchunk = a.nkb * (BKI / 16);
+    const int N = a.N, k0 = tid * E;
+    const int nchunk = a.nkb * (BKI / E);
     const bool mine = tid < nchunk;
-    float rv[16], mv[16];                                  // the first matrix's vectors do not depend on the work before
-    if (CH > 0 && mine) {
-        load16(a.p[blockIdx.y].ry, tid * 16, N, vec, rv);
-        load16(a.p[blockIdx.y].my, tid * 16, N, vec, mv);
+    HV<E> ry = zero_hv<E>(), my = zero_hv<E>(), mix = zero_hv<E>(), lw = zero_hv<E>(), lb = zero_hv<E>();
+    if (PRE && mine) {
+        const PrepProblem& p = a.p[blockIdx.y];
+        ry = load_hv<E, true>(p.ry, k0, N, vec);
+        my = load_hv<E, true>(p.my, k0, N, vec);
+        if constexpr (PRO == RWKV_PRO_LN_MIX) {
+            if (p.pro.mode != 2) mix = load_hv<E, true>(p.pro.mix, k0, N, vec);
+            lw = load_hv<E, true>(a.p[0].pro.ln_w, k0, N, vec);
+            lb = load_hv<E, true>(a.p[0].pro.ln_b, k0, N, vec);
+        }
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (t == 0 && blockIdx.y == 0)
         for (int i = tid; i < a.ntickets; i += nthr) a.tickets[i] = 0;
 
     // ---- the row, common to all matrices of the launch
-    float xx[16] = {}, prev[16] = {};
+    HV<E> xx = zero_hv<E>(), prev = zero_hv<E>();
     if constexpr (PRO == RWKV_PRO_LN_MIX) {
         // LayerNorm + token shift, rounding as rwkv_ln_mix; the previous row's output is the state or computed again
         const rwkv_mm8_seq_prologue& q = a.p[0].pro;
         const bool shift = q.sx != nullptr, own = !shift || t == 0 || q.sx_stride != 0;
         const __half* x = static_cast<const __half*>(a.p[0].x) + (long long)t * a.p[0].x_stride;
-        load16(x, k0, N, vec, xx);
-        if (shift && own) load16(static_cast<const __half*>(q.sx) + (long long)t * q.sx_stride, k0, N, vec, prev);
-        else if (shift) load16(x - a.p[0].x_stride, k0, N, vec, prev);
-        float lw[16], lb[16];
-        load16(static_cast<const __half*>(q.ln_w), k0, N, vec, lw);
-        load16(static_cast<const __half*>(q.ln_b), k0, N, vec, lb);
+        xx = load_hv<E>(x, k0, N, vec);
+        if (shift) prev = own ? load_hv<E>(static_cast<const __half*>(q.sx) + (long long)t * q.sx_stride, k0, N, vec)
+                              : load_hv<E>(x - a.p[0].x_stride, k0, N, vec);
+        if (!PRE) {
+            lw = load_hv<E, true>(q.ln_w, k0, N, vec);
+            lb = load_hv<E, true>(q.ln_b, k0, N, vec);
+        }
         float m[2] = {0.f, 0.f}, d[2] = {0.f, 0.f};
 #pragma unroll
-        for (int e = 0; e < 16; ++e) { m[0] += xx[e]; m[1] += prev[e]; }
+        for (int e = 0; e < E; ++e) { m[0] += xx[e]; m[1] += prev[e]; }
         block_reduce<2, false>(m, sh);
         m[0] /= float(N); m[1] /= float(N);
 #pragma unroll
-        for (int e = 0; e < 16; ++e)
+        for (int e = 0; e < E; ++e)
             if (k0 + e < N) {
                 d[0] = fmaf(xx[e] - m[0], xx[e] - m[0], d[0]);
                 d[1] = fmaf(prev[e] - m[1], prev[e] - m[1], d[1]);
@@ -322,34 +347,33 @@ __global__ void __launch_bounds__(MAXT) mm8_seq_i8_prep(const __grid_constant__ 
         block_reduce<2, false>(d, sh);
         const float r0 = rsqrtf(d[0] / float(N) + 1e-5f), r1 = rsqrtf(d[1] / float(N) + 1e-5f);
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
-            xx[e] = r16((xx[e] - m[0]) * r0 * lw[e] + lb[e]);
-            if (!own) prev[e] = r16((prev[e] - m[1]) * r1 * lw[e] + lb[e]);
+        for (int e = 0; e < E; ++e) {
+            xx.set(e, (xx[e] - m[0]) * r0 * lw[e] + lb[e]);
+            if (!own) prev.set(e, (prev[e] - m[1]) * r1 * lw[e] + lb[e]);
         }
         if (blockIdx.y == 0) {
-            if (q.xx_out) store16(static_cast<__half*>(q.xx_out) + (long long)t * q.xx_stride, k0, N, vec, xx);
-            if (t == a.T - 1 && q.new_state) store16(static_cast<__half*>(q.new_state), k0, N, vec, xx);
+            if (q.xx_out) store_hv<E>(static_cast<__half*>(q.xx_out) + (long long)t * q.xx_stride, k0, N, vec, xx);
+            if (t == a.T - 1 && q.new_state) store_hv<E>(q.new_state, k0, N, vec, xx);
         }
     } else if constexpr (PRO == RWKV_PRO_WKV4) {
         // one step of the RWKV-4 recurrence per row, r * wkv with the roundings of rwkv_wkv4_seq; state in place
         const rwkv_mm8_seq_prologue& q = a.p[0].pro;
         const long long at = (long long)t * N;
-        float kk[16], vv[16], rr[16], w[16], u[16], aa[16], bb[16], pp[16];
-        load16(static_cast<const __half*>(q.k) + at, k0, N, vec, kk);
-        load16(static_cast<const __half*>(q.v) + at, k0, N, vec, vv);
-        load16(static_cast<const __half*>(a.p[0].x) + (long long)t * a.p[0].x_stride, k0, N, vec, rr);
-        load16f(q.t_decay, k0, N, vec, w);
-        load16f(q.t_first, k0, N, vec, u);
-        load16f(q.aa + at, k0, N, vec, aa);
-        load16f(q.bb + at, k0, N, vec, bb);
-        load16f(q.pp + at, k0, N, vec, pp);
+        const HV<E> kk = load_hv<E>(static_cast<const __half*>(q.k) + at, k0, N, vec), vv = load_hv<E>(static_cast<const __half*>(q.v) + at, k0, N, vec);
+        const HV<E> rr = load_hv<E>(static_cast<const __half*>(a.p[0].x) + (long long)t * a.p[0].x_stride, k0, N, vec);
+        float w[E], u[E], aa[E], bb[E], pp[E];
+        load_f<E>(q.aa + at, k0, N, vec, aa);
+        load_f<E>(q.bb + at, k0, N, vec, bb);
+        load_f<E>(q.pp + at, k0, N, vec, pp);
+        load_f<E>(q.t_decay, k0, N, vec, w);
+        load_f<E>(q.t_first, k0, N, vec, u);
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
+        for (int e = 0; e < E; ++e) {
             float ww = u[e] + kk[e];
             float p = fmaxf(pp[e], ww);
             float e1 = expf(pp[e] - p), e2 = expf(ww - p);
             const float y = (e1 * aa[e] + e2 * vv[e]) / (e1 * bb[e] + e2);
-            xx[e] = k0 + e < N ? r16(rr[e] * r16(y)) : 0.f;
+            xx.set(e, k0 + e < N ? rr[e] * r16(y) : 0.f);
             ww = w[e] + pp[e];
             p = fmaxf(ww, kk[e]);
             e1 = expf(ww - p); e2 = expf(kk[e] - p);
@@ -357,29 +381,29 @@ __global__ void __launch_bounds__(MAXT) mm8_seq_i8_prep(const __grid_constant__ 
             bb[e] = e1 * bb[e] + e2;
             pp[e] = p;
         }
-        store16(q.aa + at, k0, N, vec, aa);
-        store16(q.bb + at, k0, N, vec, bb);
-        store16(q.pp + at, k0, N, vec, pp);
+        store_f<E>(q.aa + at, k0, N, vec, aa);
+        store_f<E>(q.bb + at, k0, N, vec, bb);
+        store_f<E>(q.pp + at, k0, N, vec, pp);
     } else if constexpr (PRO == RWKV_PRO_GN_GATE) {
         // group norm of each head (biased variance), ln_x in fp32, one rounding, times the gate: rwkv_v56_seq_gn_gate
         const rwkv_mm8_seq_prologue& q = a.p[0].pro;
-        float y[16], lw[16], lb[16], g[16];
-        load16f(static_cast<const float*>(a.p[0].x) + (long long)t * a.p[0].x_stride, k0, N, vec, y);
-        load16f(static_cast<const float*>(q.ln_w), k0, N, vec, lw);
-        load16f(static_cast<const float*>(q.ln_b), k0, N, vec, lb);
-        load16(static_cast<const __half*>(q.gate) + (long long)t * q.gate_stride, k0, N, vec, g);
-        const int per = q.head / 16;                       // threads of a head: 1, 2, 4 or 8 neighbouring lanes
+        float y[E], gw[E], gb[E];
+        load_f<E>(static_cast<const float*>(a.p[0].x) + (long long)t * a.p[0].x_stride, k0, N, vec, y);
+        const HV<E> g = load_hv<E>(static_cast<const __half*>(q.gate) + (long long)t * q.gate_stride, k0, N, vec);
+        load_f<E>(static_cast<const float*>(q.ln_w), k0, N, vec, gw);
+        load_f<E>(static_cast<const float*>(q.ln_b), k0, N, vec, gb);
+        const int per = q.head / E;                       // threads of a head: 1, 2, 4 or 8 neighbouring lanes
         float s = 0.f, v = 0.f;
 #pragma unroll
-        for (int e = 0; e < 16; ++e) s += y[e];
+        for (int e = 0; e < E; ++e) s += y[e];
         for (int o = per >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         const float mean = s / float(q.head);
 #pragma unroll
-        for (int e = 0; e < 16; ++e) v = fmaf(y[e] - mean, y[e] - mean, v);
+        for (int e = 0; e < E; ++e) v = fmaf(y[e] - mean, y[e] - mean, v);
         for (int o = per >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
         const float rstd = rsqrtf(v / float(q.head) + q.eps);
 #pragma unroll
-        for (int e = 0; e < 16; ++e) xx[e] = k0 + e < N ? r16(r16((y[e] - mean) * rstd * lw[e] + lb[e]) * g[e]) : 0.f;
+        for (int e = 0; e < E; ++e) xx.set(e, k0 + e < N ? r16((y[e] - mean) * rstd * gw[e] + gb[e]) * g[e] : 0.f);
     }
 
     // ---- digits, scale and sums for each matrix
@@ -387,41 +411,40 @@ __global__ void __launch_bounds__(MAXT) mm8_seq_i8_prep(const __grid_constant__ 
     const size_t plane = (size_t)a.TT * BKI;               // TT % 8 == 0: the three planes' rows share row % 8
     for (int prob = blockIdx.y; prob < a.nprob; prob += gridDim.y) {
         const PrepProblem& p = a.p[prob];
-        const __half* x = static_cast<const __half*>(p.x) + (long long)t * p.x_stride;
-        float xp[16] = {};
+        const bool have = PRE && prob == (int)blockIdx.y;  // the vectors are in registers
+        const __half* xrow = static_cast<const __half*>(p.x) + (long long)t * p.x_stride;      // RWKV_PRO_PLAIN
+        HV<E> xv = zero_hv<E>();
         float red[4] = {0.f, 0.f, 0.f, 0.f};               // maximum, SX, SXR, SXMY
         auto first = [&](int c) {
-            float xv[16];
+            const int kc = c * E;
             if constexpr (PRO == RWKV_PRO_PLAIN) {
-                load16(x, c * 16, N, vec, xv);
+                xv = load_hv<E>(xrow, kc, N, vec);
             } else if constexpr (PRO == RWKV_PRO_LN_MIX) {
-                float mix[16] = {};
-                if (p.pro.mode != 2) load16(static_cast<const __half*>(p.pro.mix), c * 16, N, vec, mix);
+                if (!have && p.pro.mode != 2) mix = load_hv<E, true>(p.pro.mix, kc, N, vec);
 #pragma unroll
-                for (int e = 0; e < 16; ++e) {
+                for (int e = 0; e < E; ++e) {
                     const float o = p.pro.mode == 2 ? xx[e]
-                                    : p.pro.mode == 0 ? r16(r16(xx[e] * mix[e]) + r16(prev[e] * r16(1.0f - mix[e])))
-                                                      : r16(xx[e] + r16(r16(prev[e] - xx[e]) * mix[e]));
-                    xv[e] = c * 16 + e < N ? o : 0.f;
+                                    : p.pro.mode == 0 ? r16(xx[e] * mix[e]) + r16(prev[e] * r16(1.0f - mix[e]))
+                                                      : xx[e] + r16(r16(prev[e] - xx[e]) * mix[e]);
+                    xv.set(e, kc + e < N ? o : 0.f);
                 }
             } else {
-#pragma unroll
-                for (int e = 0; e < 16; ++e) xv[e] = xx[e];
+                xv = xx;
             }
-            if (CH == 0 || prob != (int)blockIdx.y) {
-                load16(p.ry, c * 16, N, vec, rv);
-                load16(p.my, c * 16, N, vec, mv);
+            if (!have) {
+                ry = load_hv<E, true>(p.ry, kc, N, vec);
+                my = load_hv<E, true>(p.my, kc, N, vec);
             }
 #pragma unroll
-            for (int e = 0; e < 16; ++e) {
-                xp[e] = xv[e] * rv[e];
-                red[1] += xv[e];
-                red[2] += xp[e];
-                red[3] = fmaf(xv[e], mv[e], red[3]);
-                red[0] = fabsf(xp[e]) <= 3.0e38f ? fmaxf(red[0], fabsf(xp[e])) : INFINITY;      // fmaxf would drop a NaN
+            for (int e = 0; e < E; ++e) {
+                const float xe = xv[e], xp = xe * ry[e];
+                red[1] += xe;
+                red[2] += xp;
+                red[3] = fmaf(xe, my[e], red[3]);
+                red[0] = fabsf(xp) <= 3.0e38f ? fmaxf(red[0], fabsf(xp)) : INFINITY;      // fmaxf would drop a NaN
             }
         };
-        if constexpr (CH > 0) { if (mine) first(tid); }
+        if constexpr (!LOOP) { if (mine) first(tid); }
         else for (int c = tid; c < nchunk; c += nthr) first(c);
         block_reduce<4, true>(red, sh);
         // the power of two `up` that takes the maximum into [2^22, 2^23), or half of it if three digits would not hold it
@@ -434,27 +457,38 @@ __global__ void __launch_bounds__(MAXT) mm8_seq_i8_prep(const __grid_constant__ 
         } else if (red[0] > 0.f) {
             down = NAN;                                     // a NaN or an infinity among the activations: the row is NaN
         }
-        const bool finite = down == down;
         uint8_t* img = a.images + ((size_t)prob * a.ntt + tt) * a.nkb * (size_t)(3 * a.TT * BKI) + (size_t)ti * BKI;
         auto second = [&](int c, int& isum) {
-            if (!finite) {
+            uint32_t d[3][E / 4] = {};
 #pragma unroll
-                for (int e = 0; e < 16; ++e) xp[e] = 0.f;
+            for (int e = 0; e < E; ++e) {
+                const int q = up > 0.f ? __float2int_rn(xv[e] * ry[e] * up) : 0;
+                isum += q;
+                const int d0 = (int)(int8_t)(q & 255), q1 = (q - d0) >> 8;
+                const int d1 = (int)(int8_t)(q1 & 255), d2 = (q1 - d1) >> 8;
+                d[0][e >> 2] |= (uint32_t)(d0 & 255) << (8 * (e & 3));
+                d[1][e >> 2] |= (uint32_t)(d1 & 255) << (8 * (e & 3));
+                d[2][e >> 2] |= (uint32_t)(d2 & 255) << (8 * (e & 3));
             }
-            store_digits(xp, up, img + (size_t)(c >> 3) * (3 * plane) + (((c & 7) ^ (ti & 7)) << 4), plane, isum);
+            const int kc = c * E;
+            uint8_t* dst = img + (size_t)(kc >> 7) * (3 * plane) + ((((kc >> 4) & 7) ^ (ti & 7)) << 4) + (kc & 15);
+            typedef typename VecOf<E>::T V;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                V o;
+                memcpy(&o, d[i], sizeof(o));
+                *reinterpret_cast<V*>(dst + i * plane) = o;
+            }
         };
         long long qsum = 0;
-        if constexpr (CH > 0) {
+        if constexpr (!LOOP) {
             int isum = 0;
             if (mine) second(tid, isum);
             qsum = isum;
         } else {
             for (int c = tid; c < nchunk; c += nthr) {
-                float xv[16];
-                load16(x, c * 16, N, vec, xv);
-                load16(p.ry, c * 16, N, vec, rv);
-#pragma unroll
-                for (int e = 0; e < 16; ++e) xp[e] = xv[e] * rv[e];
+                xv = load_hv<E>(xrow, c * E, N, vec);
+                ry = load_hv<E, true>(p.ry, c * E, N, vec);
                 int isum = 0;
                 second(c, isum);
                 qsum += isum;
@@ -944,19 +978,38 @@ int rwkv_mm8_seq_i8(int nprob, const SeqI8Problem* probs, int64_t T, int64_t N, 
         }
         if (dev < 64) configured[dev] = true;
     }
-    const int nchunk = p.nkb * (BKI / 16);
-    const int threads = std::min(1024, (nchunk + 31) / 32 * 32);
-    // few rows: a block per (row, matrix), so that they run side by side; many: the row is normalised once for all matrices
-    const dim3 pgrid((unsigned)T, (unsigned)(T * nprob <= 2 * rwkv_sm_count() ? nprob : 1));
-    if (nchunk > 1024 && pro != RWKV_PRO_PLAIN) return RWKV_ERR_UNSUPPORTED;
-    auto prep = [&](auto kernel) { return rwkv_launch_pdl(kernel, pgrid, dim3(threads), 0, st, pa); };
-    const bool small = threads <= 512;
+    // Few rows: a block per (row, matrix), so that they run side by side, with as many threads as a row has groups of four.
+    // Many rows: the row is normalised once for all matrices, and as many blocks as fit an SM matter more than what one of
+    // them takes (1024 rows of 4096, LayerNorm + 2 matrices: 47 us with 2 blocks of 128 registers a thread on an SM).
+    const bool few = T * nprob <= 2 * rwkv_sm_count();
+    const dim3 pgrid((unsigned)T, (unsigned)(few ? nprob : 1));
+    const int Np = p.nkb * BKI;
+    if (pro != RWKV_PRO_PLAIN && Np > 16384) return RWKV_ERR_UNSUPPORTED;
+    const int E = (few || pro == RWKV_PRO_WKV4) && Np <= 4096 ? 4 : few && Np <= 8192 ? 8 : 16;
+    const int threads = std::min(1024, (Np / E + 31) / 32 * 32);
+    auto prep = [&](auto kernel, int n) { return rwkv_launch_pdl(kernel, pgrid, dim3(n), 0, st, pa); };
     int rc;
-    if (nchunk > 1024) rc = prep(mm8_seq_i8_prep<RWKV_PRO_PLAIN, 0, 1024>);
-    else if (pro == RWKV_PRO_LN_MIX) rc = small ? prep(mm8_seq_i8_prep<RWKV_PRO_LN_MIX, 1, 512>) : prep(mm8_seq_i8_prep<RWKV_PRO_LN_MIX, 1, 1024>);
-    else if (pro == RWKV_PRO_WKV4) rc = small ? prep(mm8_seq_i8_prep<RWKV_PRO_WKV4, 1, 512>) : prep(mm8_seq_i8_prep<RWKV_PRO_WKV4, 1, 1024>);
-    else if (pro == RWKV_PRO_GN_GATE) rc = small ? prep(mm8_seq_i8_prep<RWKV_PRO_GN_GATE, 1, 512>) : prep(mm8_seq_i8_prep<RWKV_PRO_GN_GATE, 1, 1024>);
-    else rc = prep(mm8_seq_i8_prep<RWKV_PRO_PLAIN, 1, 1024>);
+    if (pro == RWKV_PRO_PLAIN) {
+        if (few && Np <= 4096) rc = prep(mm8_seq_i8_prep<RWKV_PRO_PLAIN, 4, false, true, 1024, 2>, threads);
+        else if (few) rc = prep(mm8_seq_i8_prep<RWKV_PRO_PLAIN, 4, true, false, 1024, 2>, 1024);
+        else rc = prep(mm8_seq_i8_prep<RWKV_PRO_PLAIN, 16, true, false, 256, 4>, std::min(256, threads));
+    } else if (pro == RWKV_PRO_LN_MIX) {
+        if (E == 4) rc = prep(mm8_seq_i8_prep<RWKV_PRO_LN_MIX, 4, false, true, 1024, 2>, threads);
+        else if (E == 8) rc = prep(mm8_seq_i8_prep<RWKV_PRO_LN_MIX, 8, false, true, 1024, 1>, threads);
+        else if (threads > 512) rc = prep(mm8_seq_i8_prep<RWKV_PRO_LN_MIX, 16, false, false, 1024, 1>, threads);
+        else if (threads > 256) rc = prep(mm8_seq_i8_prep<RWKV_PRO_LN_MIX, 16, false, false, 512, 2>, threads);
+        else rc = prep(mm8_seq_i8_prep<RWKV_PRO_LN_MIX, 16, false, false, 256, 4>, threads);
+    } else if (pro == RWKV_PRO_WKV4) {
+        if (E == 4) rc = prep(mm8_seq_i8_prep<RWKV_PRO_WKV4, 4, false, true, 1024, 2>, threads);
+        else if (E == 8) rc = prep(mm8_seq_i8_prep<RWKV_PRO_WKV4, 8, false, true, 1024, 1>, threads);
+        else rc = prep(mm8_seq_i8_prep<RWKV_PRO_WKV4, 16, false, false, 1024, 1>, threads);
+    } else {
+        if (E == 4) rc = prep(mm8_seq_i8_prep<RWKV_PRO_GN_GATE, 4, false, true, 1024, 2>, threads);
+        else if (E == 8) rc = prep(mm8_seq_i8_prep<RWKV_PRO_GN_GATE, 8, false, true, 1024, 1>, threads);
+        else if (threads > 512) rc = prep(mm8_seq_i8_prep<RWKV_PRO_GN_GATE, 16, false, false, 1024, 1>, threads);
+        else if (threads > 256) rc = prep(mm8_seq_i8_prep<RWKV_PRO_GN_GATE, 16, false, false, 512, 2>, threads);
+        else rc = prep(mm8_seq_i8_prep<RWKV_PRO_GN_GATE, 16, false, false, 256, 4>, threads);
+    }
     if (rc != RWKV_OK) return rc;
     if (!p.pair) return rwkv_launch_pdl(mm8_seq_i8_kernel<1>, dim3(p.units), dim3(kThreadsI8), size_t(p.smem), st, a);
     return rwkv_launch_pdl_clustered(2, mm8_seq_i8_kernel<2>, dim3(p.units * 2), dim3(kThreadsI8), size_t(p.smem), st, a);
