@@ -134,6 +134,7 @@ SIGNATURES = {
     "rwkv_v6_att_pre": (_i32, [_i64, _i64, _i64] + [_vp] * 17),
     "rwkv_v6_token_shift": (_i32, [_i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp, _vp, _vp, _vp]),
     "rwkv_v6_decay": (_i32, [_i64, _i64, _vp, _vp, _vp, _vp, _vp, _sz, _vp, _vp]),
+    "rwkv_wkv56_one_rows": (_i32, [_i64, _i64, _i64, _vp, _vp, _vp, _vp, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     "rwkv_wkv56_one": (_i32, [_i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
 }
 

@@ -248,9 +248,11 @@ __global__ void __launch_bounds__(kT) lora_b_kernel(const LoraB b) {
 }
 
 // One-step WKV of RWKV-5.2 / RWKV-6 for one token, then group-norm (eps 64e-5) and the gate.
-// State in the model's layout [H, key j, value i] (pkg/model.py:1461-1471).  grid = H, block = 256:
+// State in the model's layout [H, key j, value i] (pkg/model.py:1461-1471).  grid = heads of all sequences, block = 256;
+// u and ln_x (and w unless every sequence has its own) are those of head % Hp.  Bound by the state's 32 KB per head of 64
+// once many sequences run at once (64 x 64 heads: 134 MB in and out):
 // thread (q, i) covers the keys j = q, q + TPI, ... of value index i (TPI = 256 / N threads per i).
-__global__ void __launch_bounds__(kT) wkv56_one_kernel(int N, const __half* __restrict__ r, const __half* __restrict__ k,
+__global__ void __launch_bounds__(kT) wkv56_one_kernel(int N, int Hp, int w_per_row, const __half* __restrict__ r, const __half* __restrict__ k,
                                                       const __half* __restrict__ v, const float* __restrict__ w,
                                                       const float* __restrict__ u, const float* s_in, float* s_out,
                                                       const float* __restrict__ lnx_w, const float* __restrict__ lnx_b,
@@ -258,7 +260,9 @@ __global__ void __launch_bounds__(kT) wkv56_one_kernel(int N, const __half* __re
     extern __shared__ float sm[];               // rr[N] kk[N] ww[N] uu[N] | acc[TPI][N]
     __shared__ float sh8[kT / 32];
     float* rr = sm; float* kk = sm + N; float* ww = sm + 2 * N; float* uu = sm + 3 * N; float* accs = sm + 4 * N;
-    const int hh = blockIdx.x, tid = threadIdx.x, c0 = hh * N;
+    const int hh = blockIdx.x, tid = threadIdx.x;
+    const long long c0 = (long long)hh * N;
+    const int p0 = (hh % Hp) * N;
     pdl_open();
     {   // the head's state (written a token ago)
         const char* base = reinterpret_cast<const char*>(s_in + (long long)hh * N * N);
@@ -268,8 +272,8 @@ __global__ void __launch_bounds__(kT) wkv56_one_kernel(int N, const __half* __re
     for (int j = tid; j < N; j += kT) {
         rr[j] = __half2float(__ldcg(r + c0 + j));
         kk[j] = __half2float(__ldcg(k + c0 + j));
-        ww[j] = __ldcg(w + c0 + j);
-        uu[j] = u[c0 + j];
+        ww[j] = __ldcg(w + (w_per_row ? c0 : (long long)p0) + j);
+        uu[j] = u[p0 + j];
     }
     __syncthreads();
     const int TPI = max(1, kT / N);
@@ -303,8 +307,8 @@ __global__ void __launch_bounds__(kT) wkv56_one_kernel(int N, const __half* __re
     const float dv = tid < N ? y - mean : 0.f;
     const float var = block_sum(dv * dv, sh8) / float(N);
     if (tid < N) {
-        const int c = c0 + tid;
-        const float o = dv * rsqrtf(var + 64e-5f) * lnx_w[c] + lnx_b[c];
+        const long long c = c0 + tid;
+        const float o = dv * rsqrtf(var + 64e-5f) * lnx_w[p0 + tid] + lnx_b[p0 + tid];
         out[c] = __float2half_rn(r16(r16(o) * __half2float(__ldcg(g + c))));
     }
 }
@@ -727,11 +731,18 @@ extern "C" int rwkv_v6_decay(int64_t D, int64_t Ld, const void* wx, const void* 
 extern "C" int rwkv_wkv56_one(int64_t H, int64_t N, const void* r, const void* k, const void* v, const float* w,
                               const float* u, const float* state, float* new_state, const float* lnx_w,
                               const float* lnx_b, const void* g, void* out, void* stream) {
-    RWKV_CHECK_ARG(H >= 1 && H <= 65535 && N >= 1 && N <= kT);
+    RWKV_CHECK_ARG(H <= 65535);
+    return rwkv_wkv56_one_rows(1, H, N, r, k, v, w, 1, u, state, new_state, lnx_w, lnx_b, g, out, stream);
+}
+
+extern "C" int rwkv_wkv56_one_rows(int64_t B, int64_t H, int64_t N, const void* r, const void* k, const void* v, const float* w,
+                                   int w_per_row, const float* u, const float* state, float* new_state, const float* lnx_w,
+                                   const float* lnx_b, const void* g, void* out, void* stream) {
+    RWKV_CHECK_ARG(B >= 1 && H >= 1 && N >= 1 && N <= kT && B * H <= INT32_MAX);
     RWKV_CHECK_ARG(r && k && v && w && u && state && new_state && lnx_w && lnx_b && g && out);
     const int TPI = kT / int(N) > 0 ? kT / int(N) : 1;
-    return rwkv_launch_pdl(wkv56_one_kernel, dim3(int(H)), dim3(kT), (4 * N + TPI * N) * sizeof(float),
-                           static_cast<cudaStream_t>(stream), int(N), static_cast<const __half*>(r),
+    return rwkv_launch_pdl(wkv56_one_kernel, dim3(unsigned(B * H)), dim3(kT), (4 * N + TPI * N) * sizeof(float),
+                           static_cast<cudaStream_t>(stream), int(N), int(H), w_per_row, static_cast<const __half*>(r),
                            static_cast<const __half*>(k), static_cast<const __half*>(v), w, u, state, new_state, lnx_w, lnx_b,
                            static_cast<const __half*>(g), static_cast<__half*>(out));
 }

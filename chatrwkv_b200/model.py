@@ -353,7 +353,6 @@ class RWKV:
         self._fork_streams = []
         self._batch_fork = os.environ.get("RWKV_B200_BATCH_FORK", "1") != "0"
         self._v6_decay_fork = os.environ.get("RWKV_B200_V6_DECAY_FORK", "1") != "0"
-        self._tile_cache = {}
         self._batch_graphs = {}
         # a matrix with more than 16384 in-features needs the decode kernel's second build: ask for it on every launch
         self._gemv_flags = _lib.MM8_WIDE_BUILD if max(a.n_ffn, a.n_att, a.n_embd) > 16384 else 0
@@ -1005,7 +1004,7 @@ class RWKV:
         st[i * 5 + 0] = new_sx
         return x + out
 
-    def _att_seq_v56(self, x, st2, i, rows=False, early=False):
+    def _att_seq_v56(self, x, st2, i, rows=False, early=False, in_place=False):
         """cuda_att_seq_v5_2 / cuda_att_seq_v6_0 (model.py:1363-1439).  `st2` = [att_xx, att_kv]; the first entry is
         replaced, the matrix state is updated in place in the model's [H, key, value] layout.  Kernels of this
         library throughout; the four small low-rank products of RWKV-6 (ranks 32..160) are plain fp16 library GEMMs
@@ -1086,21 +1085,21 @@ class RWKV:
                 k = self._mm_epi(kx, att + "key.weight", EPI_STORE, early=early)
                 v = self._mm_epi(vx, att + "value.weight", EPI_STORE, early=early)
                 g = self._mm_epi(gx, att + "gate.weight", EPI_SILU, early=early)
-        y = torch.empty((T, D), dtype=torch.float32, device=dev)
         S_in = st2[1] if st2[1].is_contiguous() else st2[1].contiguous()
-        S = torch.empty_like(S_in)                  # the caller's state stays as it is, as with the reference's copy
-        u = w[att + "time_first"].reshape(-1)
-        if rows:
-            # T sequences of one step each = T * H independent heads of one step; the per-head vectors repeat per sequence
-            u = self._tiled(att + "time_first", u, T)
-            if self.version != 6:
-                decay = self._tiled(att + "time_decay", decay, T)
-            ops.wkv56_seq(self.version == 6, T * H, S_in, r.view(1, T * D), k.view(1, T * D), v.view(1, T * D), decay.view(-1) if
-                          self.version != 6 else decay.view(1, T * D), u, y.view(1, T * D), model_layout=True, state_out=S)
-        else:
-            ops.wkv56_seq(self.version == 6, H, S_in, r, k, v, decay, u, y, model_layout=True, state_out=S)
+        # the caller's state stays as it is, as with the reference's copy (`in_place`: the batch graph owns it)
+        S = S_in if in_place else torch.empty_like(S_in)
         st2[0] = new_sx
         st2[1] = S
+        u = w[att + "time_first"].reshape(-1)
+        if rows:    # T sequences of one step each: recurrence, group norm and gate per head as in one-token decode
+            out = h(T, D)
+            check(L.rwkv_wkv56_one_rows(T, H, N, r.data_ptr(), k.data_ptr(), v.data_ptr(), decay.data_ptr(),
+                                        1 if self.version == 6 else 0, u.data_ptr(), S_in.data_ptr(), S.data_ptr(),
+                                        w[att + "ln_x.weight"].data_ptr(), w[att + "ln_x.bias"].data_ptr(), g.data_ptr(),
+                                        out.data_ptr(), stream), "wkv56_one_rows")
+            return self._mm_epi(out, att + "output.weight", EPI_RESIDUAL, aux=x, out=x)
+        y = torch.empty((T, D), dtype=torch.float32, device=dev)
+        ops.wkv56_seq(self.version == 6, H, S_in, r, k, v, decay, u, y, model_layout=True, state_out=S)
         arr, _ = self._seq_group(PRO_GN_GATE, [(att + "output.weight", EPI_RESIDUAL)], ln=(att + "ln_x.weight", att + "ln_x.bias"))
         if arr is not None and not early:
             q = arr[0]
@@ -1112,14 +1111,6 @@ class RWKV:
         check(L.rwkv_v56_seq_gn_gate(T, H, N, y.data_ptr(), w[att + "ln_x.weight"].data_ptr(), w[att + "ln_x.bias"].data_ptr(),
                                      g.data_ptr(), out.data_ptr(), 64e-5, stream), "gn_gate")
         return self._mm_epi(out, att + "output.weight", EPI_RESIDUAL, aux=x, out=x, early=early)
-
-    def _tiled(self, name, t, reps):
-        """A per-head / per-channel model vector repeated for `reps` sequences (cached: made once per batch size)."""
-        key = (name, reps)
-        c = self._tile_cache.get(key)
-        if c is None:
-            c = self._tile_cache[key] = t.reshape(-1).repeat(reps).contiguous()
-        return c
 
     def _ffn_seq(self, x, sx, i, rows=False, early=False):
         """ffn_seq / ffn_seq_v6 (model.py:995-1004, 1019-1029)."""
@@ -1171,7 +1162,8 @@ class RWKV:
         state returned by an earlier call (or by zero_batch_state / stack_states).  Returns (logits fp32 [B, V],
         batch state).  The B sequences are the rows of the tensor-core mm8_seq kernel, so the packed weights are
         streamed once per step for all of them; every sequence follows the arithmetic of the prefill path with T = 1.
-        The RWKV-4 WKV states (aa, bb, pp) are updated in place, everything else is returned in new tensors."""
+        The RWKV-4 WKV states (aa, bb, pp) are updated in place, everything else is returned in new tensors (with
+        graphs, in the tensors that _forward_batch_graph names)."""
         if self._world > 1:
             raise NotImplementedError("forward_batch: single-GPU models only")
         with torch.no_grad(), torch.cuda.device(self.device):
@@ -1200,7 +1192,7 @@ class RWKV:
             torch.cuda.synchronize(self.device)
             graph = torch.cuda.CUDAGraph()
             with torch.cuda.graph(graph, stream=side):
-                g.logits, g.out = self._forward_batch_eager(g.tok, g.inp)
+                g.logits, g.out = self._forward_batch_eager(g.tok, g.inp, in_place=True)
             # the previous step's outputs become the next step's inputs (entries updated in place are their own output)
             moved = [(i, o) for i, o in zip(g.inp, g.out) if i is not o]
             g.graph, g.moved = graph, moved
@@ -1220,7 +1212,7 @@ class RWKV:
         g.graph.replay()
         return g.logits.clone(), list(g.out)
 
-    def _forward_batch_eager(self, idx, state):
+    def _forward_batch_eager(self, idx, state, in_place=False):
         with torch.no_grad():
             w, a = self.w, self.args
             B = idx.numel()
@@ -1232,7 +1224,7 @@ class RWKV:
                     x, state[i * 5 + 4] = self._ffn_seq(x, state[i * 5 + 4], i, rows=True)
                 else:
                     st2 = [state[i * 3 + 0], state[i * 3 + 1]]
-                    x = self._att_seq_v56(x, st2, i, rows=True)
+                    x = self._att_seq_v56(x, st2, i, rows=True, in_place=in_place)
                     state[i * 3 + 0], state[i * 3 + 1] = st2
                     x, state[i * 3 + 2] = self._ffn_seq(x, state[i * 3 + 2], i, rows=True)
             return self._head_rows(x).float(), state

@@ -556,6 +556,11 @@ int rwkv_v6_decay(int64_t D, int64_t Ld, const void* wx, const void* td_w1, cons
 int rwkv_wkv56_one(int64_t H, int64_t N, const void* r, const void* k, const void* v, const float* w,
                    const float* u, const float* state, float* new_state, const float* lnx_w,
                    const float* lnx_b, const void* g, void* out, void* stream);
+/* The same for B sequences at once: r, k, v, g, out [B, H*N], states [B, H, N, N] (new_state may be state); u, lnx_w, lnx_b
+ * [H*N]; w [B, H*N] with w_per_row (RWKV-6), else [H*N]. */
+int rwkv_wkv56_one_rows(int64_t B, int64_t H, int64_t N, const void* r, const void* k, const void* v, const float* w,
+                        int w_per_row, const float* u, const float* state, float* new_state, const float* lnx_w,
+                        const float* lnx_b, const void* g, void* out, void* stream);
 
 /* ---------------------------------------------------------------------------------------
  * Token sampling on the device — PIPELINE.sample_logits and the penalty bookkeeping of
