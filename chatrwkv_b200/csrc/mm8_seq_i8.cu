@@ -187,10 +187,10 @@ __device__ __forceinline__ void tmem_ld8(int (&v)[8], uint32_t addr) {
 // ---- preparation: x' as digit planes, the row sums and scales ------------------------------------
 // One block per row (or per row and matrix); a thread owns E neighbouring k.  What produces the row (LayerNorm + token
 // shift, the one-step WKV, group norm + gate) runs in the same pass.  A block is a chain of latencies: one trip to memory,
-// two to four reductions, and the code itself, which the streamed weights have evicted (with 16 k a thread a launch of 16
-// rows took 10 us after its wait, 2.5 us when repeated alone).  So few rows run with E = 4: short code, and the weights'
-// vectors fetched before the dependency wait.  With many rows what counts is how many blocks an SM holds: E = 16, rows
-// kept as fp16, the vectors read when needed.
+// two to four reductions, and vectors and code that the streamed weights have evicted.  Few rows run with the weights'
+// vectors fetched before the dependency wait and E = 8 (16 rows of 4096, LayerNorm + mix, from the wait to the end, in a 7B
+// layer: 10 us with E = 16, 9 us with E = 4 whose 32 warps wait for each other in every reduction, 6.5 us with E = 8).
+// With many rows what counts is how many blocks an SM holds: E = 16, rows kept as fp16, the vectors read when needed.
 template <int E> struct HV {                     // E fp16 values
     __half2 h[E / 2];
     __device__ __forceinline__ float operator[](int e) const { return (e & 1) ? __high2float(h[e >> 1]) : __low2float(h[e >> 1]); }
@@ -459,16 +459,22 @@ __global__ void __launch_bounds__(MAXT, MINB) mm8_seq_i8_prep(const __grid_const
         }
         uint8_t* img = a.images + ((size_t)prob * a.ntt + tt) * a.nkb * (size_t)(3 * a.TT * BKI) + (size_t)ti * BKI;
         auto second = [&](int c, int& isum) {
-            uint32_t d[3][E / 4] = {};
+            // balanced base-256 digits: the bytes of q + 128 * (1 + 256 + 65536), each minus 128
+            uint32_t d[3][E / 4];
 #pragma unroll
-            for (int e = 0; e < E; ++e) {
-                const int q = up > 0.f ? __float2int_rn(xv[e] * ry[e] * up) : 0;
-                isum += q;
-                const int d0 = (int)(int8_t)(q & 255), q1 = (q - d0) >> 8;
-                const int d1 = (int)(int8_t)(q1 & 255), d2 = (q1 - d1) >> 8;
-                d[0][e >> 2] |= (uint32_t)(d0 & 255) << (8 * (e & 3));
-                d[1][e >> 2] |= (uint32_t)(d1 & 255) << (8 * (e & 3));
-                d[2][e >> 2] |= (uint32_t)(d2 & 255) << (8 * (e & 3));
+            for (int e = 0; e < E; e += 4) {
+                uint32_t u[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int q = up > 0.f ? __float2int_rn(xv[e + i] * ry[e + i] * up) : 0;
+                    isum += q;
+                    u[i] = (uint32_t)(q + 0x808080);
+                }
+                const uint32_t lo01 = __byte_perm(u[0], u[1], 0x5140), lo23 = __byte_perm(u[2], u[3], 0x5140);
+                const uint32_t hi01 = __byte_perm(u[0], u[1], 0x0062), hi23 = __byte_perm(u[2], u[3], 0x0062);
+                d[0][e >> 2] = __byte_perm(lo01, lo23, 0x5410) ^ 0x80808080u;
+                d[1][e >> 2] = __byte_perm(lo01, lo23, 0x7632) ^ 0x80808080u;
+                d[2][e >> 2] = __byte_perm(hi01, hi23, 0x5410) ^ 0x80808080u;
             }
             const int kc = c * E;
             uint8_t* dst = img + (size_t)(kc >> 7) * (3 * plane) + ((((kc >> 4) & 7) ^ (ti & 7)) << 4) + (kc & 15);
@@ -499,11 +505,15 @@ __global__ void __launch_bounds__(MAXT, MINB) mm8_seq_i8_prep(const __grid_const
         __syncthreads();
         if (lane == 0) shq[warp] = qsum;
         __syncthreads();
-        if (tid == 0) {
-            RowConst rc;
-            rc.scale = down; rc.sx = red[1]; rc.sxr = red[2]; rc.sxmy = red[3]; rc.corr = 0; rc.pad = 0;
-            for (int i = 0; i < nwarp; ++i) rc.corr -= 128 * shq[i];
-            a.consts[(size_t)prob * a.T + t] = rc;
+        if (warp == 0) {
+            qsum = lane < nwarp ? shq[lane] : 0;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) qsum += __shfl_xor_sync(0xffffffffu, qsum, o);
+            if (lane == 0) {
+                RowConst rc;
+                rc.scale = down; rc.sx = red[1]; rc.sxr = red[2]; rc.sxmy = red[3]; rc.corr = -128 * qsum; rc.pad = 0;
+                a.consts[(size_t)prob * a.T + t] = rc;
+            }
         }
     }
 }
@@ -978,20 +988,21 @@ int rwkv_mm8_seq_i8(int nprob, const SeqI8Problem* probs, int64_t T, int64_t N, 
         }
         if (dev < 64) configured[dev] = true;
     }
-    // Few rows: a block per (row, matrix), so that they run side by side, with as many threads as a row has groups of four.
+    // Few rows: a block per (row, matrix), so that they run side by side (E: see above).
     // Many rows: the row is normalised once for all matrices, and as many blocks as fit an SM matter more than what one of
     // them takes (1024 rows of 4096, LayerNorm + 2 matrices: 47 us with 2 blocks of 128 registers a thread on an SM).
     const bool few = T * nprob <= 2 * rwkv_sm_count();
     const dim3 pgrid((unsigned)T, (unsigned)(few ? nprob : 1));
     const int Np = p.nkb * BKI;
     if (pro != RWKV_PRO_PLAIN && Np > 16384) return RWKV_ERR_UNSUPPORTED;
-    const int E = (few || pro == RWKV_PRO_WKV4) && Np <= 4096 ? 4 : few && Np <= 8192 ? 8 : 16;
+    const int E = (few || pro == RWKV_PRO_WKV4) && Np <= 1024 ? 4 : (few || pro == RWKV_PRO_WKV4) && Np <= 8192 ? 8 : 16;
     const int threads = std::min(1024, (Np / E + 31) / 32 * 32);
     auto prep = [&](auto kernel, int n) { return rwkv_launch_pdl(kernel, pgrid, dim3(n), 0, st, pa); };
     int rc;
     if (pro == RWKV_PRO_PLAIN) {
-        if (few && Np <= 4096) rc = prep(mm8_seq_i8_prep<RWKV_PRO_PLAIN, 4, false, true, 1024, 2>, threads);
-        else if (few) rc = prep(mm8_seq_i8_prep<RWKV_PRO_PLAIN, 4, true, false, 1024, 2>, 1024);
+        if (E == 4) rc = prep(mm8_seq_i8_prep<RWKV_PRO_PLAIN, 4, false, true, 1024, 2>, threads);
+        else if (E == 8) rc = prep(mm8_seq_i8_prep<RWKV_PRO_PLAIN, 8, false, true, 1024, 1>, threads);
+        else if (few) rc = prep(mm8_seq_i8_prep<RWKV_PRO_PLAIN, 8, true, false, 1024, 1>, 1024);
         else rc = prep(mm8_seq_i8_prep<RWKV_PRO_PLAIN, 16, true, false, 256, 4>, std::min(256, threads));
     } else if (pro == RWKV_PRO_LN_MIX) {
         if (E == 4) rc = prep(mm8_seq_i8_prep<RWKV_PRO_LN_MIX, 4, false, true, 1024, 2>, threads);

@@ -34,7 +34,7 @@ def _close(got, want):
     assert (got.float() - want.float()).pow(2).mean().sqrt() <= 2 ** -10 * rms
 
 
-@pytest.mark.parametrize("T,N", [(2, 300), (16, 768), (40, 4096), (5, 5120), (120, 8320), (300, 1024)])
+@pytest.mark.parametrize("T,N", [(2, 300), (16, 768), (40, 4096), (5, 5120), (120, 8064), (300, 1024)])
 @pytest.mark.parametrize("mode,rows", [(0, True), (0, False), (1, False), (2, True)])
 def test_layer_norm_mix(ops, T, N, mode, rows):
     from chatrwkv_b200 import _lib
