@@ -347,9 +347,9 @@ __global__ void __launch_bounds__(MAXT, MINB) mm8_seq_i8_prep(const __grid_const
         block_reduce<2, false>(d, sh);
         const float r0 = rsqrtf(d[0] / float(N) + 1e-5f), r1 = rsqrtf(d[1] / float(N) + 1e-5f);
 #pragma unroll
-        for (int e = 0; e < E; ++e) {
-            xx.set(e, (xx[e] - m[0]) * r0 * lw[e] + lb[e]);
-            if (!own) prev.set(e, (prev[e] - m[1]) * r1 * lw[e] + lb[e]);
+        for (int e = 0; e < E; e += 2) {
+            xx.h[e >> 1] = __floats2half2_rn((xx[e] - m[0]) * r0 * lw[e] + lb[e], (xx[e + 1] - m[0]) * r0 * lw[e + 1] + lb[e + 1]);
+            if (!own) prev.h[e >> 1] = __floats2half2_rn((prev[e] - m[1]) * r1 * lw[e] + lb[e], (prev[e + 1] - m[1]) * r1 * lw[e + 1] + lb[e + 1]);
         }
         if (blockIdx.y == 0) {
             if (q.xx_out) store_hv<E>(static_cast<__half*>(q.xx_out) + (long long)t * q.xx_stride, k0, N, vec, xx);
@@ -421,13 +421,13 @@ __global__ void __launch_bounds__(MAXT, MINB) mm8_seq_i8_prep(const __grid_const
                 xv = load_hv<E>(xrow, kc, N, vec);
             } else if constexpr (PRO == RWKV_PRO_LN_MIX) {
                 if (!have && p.pro.mode != 2) mix = load_hv<E, true>(p.pro.mix, kc, N, vec);
+                // every fp16 operation of the reference rounds once, as these do (_rn: never contracted)
+                const __half2 one = __float2half2_rn(1.f);
 #pragma unroll
-                for (int e = 0; e < E; ++e) {
-                    const float o = p.pro.mode == 2 ? xx[e]
-                                    : p.pro.mode == 0 ? r16(xx[e] * mix[e]) + r16(prev[e] * r16(1.0f - mix[e]))
-                                                      : xx[e] + r16(r16(prev[e] - xx[e]) * mix[e]);
-                    xv.set(e, kc + e < N ? o : 0.f);
-                }
+                for (int i = 0; i < E / 2; ++i)
+                    xv.h[i] = p.pro.mode == 2 ? xx.h[i]
+                              : p.pro.mode == 0 ? __hadd2_rn(__hmul2_rn(xx.h[i], mix.h[i]), __hmul2_rn(prev.h[i], __hsub2_rn(one, mix.h[i])))
+                                                : __hadd2_rn(xx.h[i], __hmul2_rn(__hsub2_rn(prev.h[i], xx.h[i]), mix.h[i]));
             } else {
                 xv = xx;
             }
