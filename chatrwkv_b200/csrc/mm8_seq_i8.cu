@@ -920,7 +920,9 @@ int rwkv_mm8_seq_i8(int nprob, const SeqI8Problem* probs, int64_t T, int64_t N, 
         M[i] = q.M;
     }
     if (encode_fn() == nullptr) return RWKV_ERR_UNSUPPORTED;
-    const Plan p = make_plan(nprob, T, N, M, g_i8_form);
+    static int use_pair = -1;            // RWKV_B200_SEQ_PAIR=0: never the CTA-pair form (same results)
+    if (use_pair < 0) { const char* e = getenv("RWKV_B200_SEQ_PAIR"); use_pair = (e != nullptr && e[0] == '0') ? 0 : 1; }
+    const Plan p = make_plan(nprob, T, N, M, use_pair ? g_i8_form : 1);
     if (workspace == nullptr || workspace_bytes < p.bytes) return RWKV_ERR_WORKSPACE;
     RWKV_CHECK_ALIGN(workspace, 256);
     uint8_t* ws = static_cast<uint8_t*>(workspace);

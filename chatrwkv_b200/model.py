@@ -1196,6 +1196,7 @@ class RWKV:
             # the previous step's outputs become the next step's inputs (entries updated in place are their own output)
             moved = [(i, o) for i, o in zip(g.inp, g.out) if i is not o]
             g.graph, g.moved = graph, moved
+            g.scratch = list(ops._workspaces.values())     # the graph's launches hold their addresses: alive as long as it is
             self._batch_graphs[B] = g
             state_is_ours = False
         else:
