@@ -43,7 +43,6 @@ __global__ void __launch_bounds__(kWkv4Threads) wkv4_summary_kernel(int T, int C
                                                                     const float* __restrict__ pp_, float* __restrict__ summ,
                                                                     float* __restrict__ init) {
     const int c = blockIdx.x * kWkv4Threads + threadIdx.x, chunk = blockIdx.y, b = blockIdx.z;
-    asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
     if (c >= C) return;
     if (chunk == 0) {
         float* ini = init + (size_t)b * 3 * C;
@@ -56,12 +55,12 @@ __global__ void __launch_bounds__(kWkv4Threads) wkv4_summary_kernel(int T, int C
     Wkv4State s = {0.f, 0.f, -1e30f};
     const int n = t1 - t0;
     int t = 0;
-    for (; t + 8 <= n; t += 8) {
-        float kk[8], vv[8];
+    for (; t + 4 <= n; t += 4) {
+        float kk[4], vv[4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) { kk[i] = to_f32<F>(k[(size_t)(t + i) * C]); vv[i] = to_f32<F>(v[(size_t)(t + i) * C]); }
+        for (int i = 0; i < 4; ++i) { kk[i] = to_f32<F>(k[(size_t)(t + i) * C]); vv[i] = to_f32<F>(v[(size_t)(t + i) * C]); }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) wkv4_step(s, w, kk[i], vv[i]);
+        for (int i = 0; i < 4; ++i) wkv4_step(s, w, kk[i], vv[i]);
     }
     for (; t < n; ++t) wkv4_step(s, w, to_f32<F>(k[(size_t)t * C]), to_f32<F>(v[(size_t)t * C]));
     float* out = summ + ((size_t)b * NC + chunk) * 3 * C;
@@ -75,7 +74,6 @@ __global__ void __launch_bounds__(kWkv4Threads) wkv4_apply_kernel(int T, int C, 
                                                                   float* aa_, float* bb_, float* pp_,
                                                                   const float* __restrict__ summ, const float* __restrict__ init) {
     const int c = blockIdx.x * kWkv4Threads + threadIdx.x, chunk = blockIdx.y, b = blockIdx.z;
-    asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
     if (c >= C) return;
     const float w = w_[c], u = u_[c];
     Wkv4State s;
@@ -85,24 +83,15 @@ __global__ void __launch_bounds__(kWkv4Threads) wkv4_apply_kernel(int T, int C, 
         const float* ini = init + (size_t)b * 3 * C;
         s.aa = ini[c]; s.bb = ini[C + c]; s.pp = ini[2 * C + c];
         const float wl = w * float(Lc);
-        const float* sm = summ + (size_t)b * NC * 3 * C + c;
-        for (int j0 = 0; j0 < chunk; j0 += 8) { // state after chunk j = e^{w Lc} state + summary_j; eight summaries in flight
-            float sa[8], sb[8], sp[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float* q = sm + (size_t)min(j0 + i, chunk - 1) * 3 * C;
-                sa[i] = q[0]; sb[i] = q[C]; sp[i] = q[2 * C];
-            }
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                if (j0 + i >= chunk) break;
-                const float ww = wl + s.pp;
-                const float p = fmaxf(ww, sp[i]);
-                const float e1 = expf(ww - p), e2 = expf(sp[i] - p);
-                s.aa = e1 * s.aa + e2 * sa[i];
-                s.bb = e1 * s.bb + e2 * sb[i];
-                s.pp = p;
-            }
+        for (int j = 0; j < chunk; ++j) {       // state after chunk j = e^{w Lc} state + summary_j
+            const float* sm = summ + ((size_t)b * NC + j) * 3 * C;
+            const float sa = sm[c], sb = sm[C + c], sp = sm[2 * C + c];
+            const float ww = wl + s.pp;
+            const float p = fmaxf(ww, sp);
+            const float e1 = expf(ww - p), e2 = expf(sp - p);
+            s.aa = e1 * s.aa + e2 * sa;
+            s.bb = e1 * s.bb + e2 * sb;
+            s.pp = p;
         }
     }
     const int t0 = chunk * Lc, t1 = min(T, t0 + Lc);
@@ -113,15 +102,15 @@ __global__ void __launch_bounds__(kWkv4Threads) wkv4_apply_kernel(int T, int C, 
     F* y = y_ + base;
     const int n = t1 - t0;
     int t = 0;
-    for (; t + 8 <= n; t += 8) {
-        float kk[8], vv[8], rr[8];
+    for (; t + 4 <= n; t += 4) {
+        float kk[4], vv[4], rr[4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < 4; ++i) {
             kk[i] = to_f32<F>(k[(size_t)(t + i) * C]); vv[i] = to_f32<F>(v[(size_t)(t + i) * C]);
             rr[i] = MULR ? to_f32<F>(r[(size_t)(t + i) * C]) : 1.f;
         }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < 4; ++i) {
             const float ww = u + kk[i];
             const float p = fmaxf(s.pp, ww);
             const float e1 = expf(s.pp - p), e2 = expf(ww - p);
@@ -495,11 +484,13 @@ static int wkv4_launch(int64_t B, int64_t T, int64_t C, const float* w, const fl
     const dim3 grid((unsigned)((C + kWkv4Threads - 1) / kWkv4Threads), (unsigned)NC, (unsigned)B);
     if (NC > 1) {
         const dim3 g1(grid.x, (unsigned)(NC - 1), grid.z);
-        const int rc = rwkv_launch_pdl(wkv4_summary_kernel<F>, g1, dim3(kWkv4Threads), 0, st, int(T), int(C), Lc, NC, w, k, v, aa, bb, pp, summ, init);
-        if (rc != RWKV_OK) return rc;
+        wkv4_summary_kernel<F><<<g1, kWkv4Threads, 0, st>>>(int(T), int(C), Lc, NC, w, k, v, aa, bb, pp, summ, init);
     }
-    return rwkv_launch_pdl(r != nullptr ? wkv4_apply_kernel<F, true> : wkv4_apply_kernel<F, false>, grid, dim3(kWkv4Threads), 0, st, int(T),
-                           int(C), Lc, NC, w, u, k, v, r, y, aa, bb, pp, summ, init);
+    if (r != nullptr)
+        wkv4_apply_kernel<F, true><<<grid, kWkv4Threads, 0, st>>>(int(T), int(C), Lc, NC, w, u, k, v, r, y, aa, bb, pp, summ, init);
+    else
+        wkv4_apply_kernel<F, false><<<grid, kWkv4Threads, 0, st>>>(int(T), int(C), Lc, NC, w, u, k, v, r, y, aa, bb, pp, summ, init);
+    return rwkv_launch_status();
 }
 
 extern "C" int rwkv_wkv4_seq(int64_t B, int64_t T, int64_t C, const float* w, const float* u,
