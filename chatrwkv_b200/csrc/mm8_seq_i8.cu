@@ -24,6 +24,9 @@
 //              stores in 16-byte pieces of rows
 //   warp 16    TMEM allocation; tcgen05.mma and tcgen05.commit
 //   warp 17    TMA loads (W ahead of the dependency wait: it was written before the launch)
+// Bound by HBM up to about 64 rows and by the int8 tensor rate above 200 (760 clocks per K block of a pair's 256 x 128
+// tile, 768 of tensor work).  Operator alone, operand pass included, fp16 path -> this one, (4096, 4096) / (4096, 16384) /
+// (16384, 4096): 16 rows 16.7 -> 12.8 / 38.9 -> 16.4 / 49.3 -> 23.4 us, 1024 rows 67 -> 48 / 248 -> 135 / 245 -> 176 us.
 // Every wait is bounded: on give-up the CTA raises an error word, skips the rest of its work and returns.
 #include "common.cuh"
 #include "seq_epi.cuh"
@@ -848,6 +851,8 @@ Plan make_plan(int nprob, int64_t T, int64_t N, const int64_t* M, int force) {
     p.nkb = int((N + BKI - 1) / BKI);
     p.ntt = int((T + kMaxTT - 1) / kMaxTT);
     const int per = int((T + p.ntt - 1) / p.ntt);
+    // Pairs halve the token planes each CTA fetches and reads; up to 32 rows these are small and single CTAs spread a matrix
+    // over twice as many units (4096 x 4096: 16 rows 13.9 against 15.0 us, 64 rows equal, 1024 rows 64 against 56 us).
     p.pair = force == 1 ? 0 : force == 2 ? 1 : (per > 32 ? 1 : 0);
     const int unit = p.pair ? 32 : 16;
     p.TT = (per + unit - 1) / unit * unit;
