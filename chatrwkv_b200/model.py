@@ -891,8 +891,9 @@ class RWKV:
 
     def _seq_group(self, kind, jobs, mode=0, ln=None, mixes=None):
         """The table of a launch of 1..4 int8 matrices (rwkv_mm8_seq_batch) with what the model fixes, and its length:
-        `jobs` = [(name, epilogue)], `ln` = the names of the norm's weight and bias, `mixes` = names.  Made once; the
-        caller sets the activations' addresses.  (None, 0) when a matrix is kept in fp16 or split over ranks."""
+        `jobs` = [(name, epilogue)], `ln` = the names of the norm's weight and bias, `mixes` = names.  The constant part is
+        made once; every call gets a copy of its own, in which it sets the activations' addresses (calls of several threads
+        may be filling theirs at the same time).  (None, 0) when a matrix is kept in fp16 or split over ranks."""
         key = jobs[0][0], kind
         t = self._seq_tables.get(key)
         if t is None:
@@ -912,7 +913,8 @@ class RWKV:
                 if mixes is not None:
                     q.mix = w[mixes[i]].data_ptr()
             t = self._seq_tables[key] = (arr, len(jobs))
-        return t
+        const, n = t
+        return (type(const).from_buffer_copy(const), n) if n else t
 
     def _ln_mix_group(self, x, sx, rows, jobs, mode, ln, mixes):
         """LayerNorm, token shift and the matmuls of the mixes as two launches (operands, matmuls).  Returns the outputs and

@@ -1,0 +1,55 @@
+"""The tables of the grouped prompt launches (RWKV._seq_group): host logic, run without a GPU on a stub of the launch."""
+import threading
+import time
+
+import pytest
+import torch
+
+from chatrwkv_b200 import _lib, ops
+from chatrwkv_b200.model import RWKV
+
+N, M = 32, 16
+
+
+@pytest.fixture
+def model():
+    m = RWKV.__new__(RWKV)
+    m._world, m._seq_tables, m._mm = 1, {}, {}
+    m.w = {"ln.weight": torch.ones(N, dtype=torch.float16), "ln.bias": torch.zeros(N, dtype=torch.float16)}
+    for name in ("r", "k"):
+        m.w["mix_" + name] = torch.rand(N).half()
+        m.w[name] = torch.zeros((N, M), dtype=torch.uint8)
+        for s, n in (("_mx", M), ("_rx", M), ("_my", N), ("_ry", N)):
+            m.w[name + s] = torch.zeros(n, dtype=torch.float16)
+    return m
+
+
+def _group(model, x, sx):
+    return model._ln_mix_group(x, sx, False, [("r", _lib.EPI_SIGMOID), ("k", _lib.EPI_STORE)], 0, ("ln.weight", "ln.bias"),
+                               ["mix_r", "mix_k"])
+
+
+def test_threads_launch_with_their_own_pointers(model, monkeypatch):
+    """Calls that overlap in time (the launch lets other threads run) never see each other's activations."""
+    mine, wrong = threading.local(), []
+
+    def launch(arr, n, T, D, device):
+        for _ in range(3):
+            x, sx = mine.now
+            if any(q.x != x.data_ptr() for q in arr) or arr[0].sx != sx.data_ptr():
+                wrong.append(T)
+            time.sleep(0)
+        return True
+    monkeypatch.setattr(ops, "mm8_seq_batch", launch)
+
+    def work(T):
+        for _ in range(200):
+            mine.now = torch.zeros((T, N), dtype=torch.float16), torch.zeros(N, dtype=torch.float16)
+            outs, _ = _group(model, *mine.now)
+            assert [tuple(o.shape) for o in outs] == [(T, M)] * 2
+    threads = [threading.Thread(target=work, args=(T,)) for T in (3, 5, 9, 17)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
