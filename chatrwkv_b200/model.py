@@ -891,9 +891,10 @@ class RWKV:
 
     def _seq_group(self, kind, jobs, mode=0, ln=None, mixes=None):
         """The table of a launch of 1..4 int8 matrices (rwkv_mm8_seq_batch) with what the model fixes, and its length:
-        `jobs` = [(name, epilogue)], `ln` = the names of the norm's weight and bias, `mixes` = names.  The constant part is
-        made once; every call gets a copy of its own, in which it sets the activations' addresses (calls of several threads
-        may be filling theirs at the same time).  (None, 0) when a matrix is kept in fp16 or split over ranks."""
+        `jobs` = [(name, epilogue)], `ln` = the names of the norm's weight and bias, `mixes` = names.  The matrices' part is
+        made once (`_scales` keeps their tensors); every call gets a copy of its own, in which it sets the activations'
+        addresses (calls of several threads may be filling theirs at the same time), with the norm and the mixes as `self.w`
+        has them now.  (None, 0) when a matrix is kept in fp16 or split over ranks."""
         key = jobs[0][0], kind
         t = self._seq_tables.get(key)
         if t is None:
@@ -908,13 +909,17 @@ class RWKV:
                 q.w, q.w_stride, q.M = wq.data_ptr(), wq.stride(0), wq.shape[1]
                 q.mx, q.rx, q.my, q.ry = mx.data_ptr(), rx.data_ptr(), my.data_ptr(), ry.data_ptr()
                 q.epilogue, q.out_scale, q.kind, q.mode = epi, 1.0, kind, mode
-                if ln is not None:
-                    q.ln_w, q.ln_b = w[ln[0]].data_ptr(), w[ln[1]].data_ptr()
-                if mixes is not None:
-                    q.mix = w[mixes[i]].data_ptr()
             t = self._seq_tables[key] = (arr, len(jobs))
         const, n = t
-        return (type(const).from_buffer_copy(const), n) if n else t
+        if not n:
+            return t
+        arr = type(const).from_buffer_copy(const)
+        if ln is not None:
+            arr[0].ln_w, arr[0].ln_b = self.w[ln[0]].data_ptr(), self.w[ln[1]].data_ptr()
+        if mixes is not None:
+            for q, name in zip(arr, mixes):
+                q.mix = self.w[name].data_ptr()
+        return arr, n
 
     def _ln_mix_group(self, x, sx, rows, jobs, mode, ln, mixes):
         """LayerNorm, token shift and the matmuls of the mixes as two launches (operands, matmuls).  Returns the outputs and

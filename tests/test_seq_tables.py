@@ -53,3 +53,23 @@ def test_threads_launch_with_their_own_pointers(model, monkeypatch):
     for t in threads:
         t.join()
     assert not wrong
+
+
+def test_replaced_norms_and_mixes_are_seen(model, monkeypatch):
+    """An entry of `model.w` that a program replaces after the first prompt: the next launch reads the new tensor (the old one's
+    memory may be gone)."""
+    seen = []
+
+    def launch(arr, n, T, D, device):
+        seen.append([arr[0].ln_w, arr[0].ln_b] + [q.mix for q in arr])
+        return True
+    monkeypatch.setattr(ops, "mm8_seq_batch", launch)
+    x, sx = torch.zeros((4, N), dtype=torch.float16), torch.zeros(N, dtype=torch.float16)
+    keep = []
+    for _ in range(2):
+        _group(model, x, sx)
+        names = ("ln.weight", "ln.bias", "mix_r", "mix_k")
+        assert seen[-1] == [model.w[k].data_ptr() for k in names]
+        for k in names:
+            keep.append(model.w[k])
+            model.w[k] = model.w[k].clone()
