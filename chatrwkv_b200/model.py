@@ -974,6 +974,7 @@ class RWKV:
             arr, _ = self._seq_group(PRO_WKV4, [(att + "output.weight", EPI_RESIDUAL)]) if rows else (None, 0)
             if arr is not None:     # T sequences of one step each: the recurrence runs in the launch that prepares the operand
                 aa, b_, pp = st[i * 5 + 1:i * 5 + 4]
+                ops._require(all(t.dtype == torch.float32 for t in (aa, b_, pp)), "w, u and the state must be fp32")
                 ops._require(all(t.is_contiguous() for t in (aa, b_, pp)), "wkv needs contiguous tensors")
                 q = arr[0]
                 q.x, q.x_stride, q.k, q.v = r.data_ptr(), r.stride(0), k.data_ptr(), v.data_ptr()

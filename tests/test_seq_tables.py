@@ -73,3 +73,27 @@ def test_replaced_norms_and_mixes_are_seen(model, monkeypatch):
         for k in names:
             keep.append(model.w[k])
             model.w[k] = model.w[k].clone()
+
+
+def test_batched_rwkv4_step_refuses_states_that_are_not_fp32(monkeypatch):
+    """The recurrence inside the operand pass reads and writes fp32: a program that stores its sessions in fp16 gets an error."""
+    m = RWKV.__new__(RWKV)
+    m._world, m._seq_tables, m._mm, m.args = 1, {}, {}, None
+    bb, att = "blocks.0.", "blocks.0.att."
+    m.w = {bb + "ln1.weight": torch.ones(N).half(), bb + "ln1.bias": torch.zeros(N).half(), att + "time_decay": torch.zeros(N),
+           att + "time_first": torch.zeros(N)}
+    for n in ("k", "v", "r"):
+        m.w[att + "time_mix_" + n] = torch.rand(N).half()
+    for n in ("receptance", "key", "value", "output"):
+        m.w[att + n + ".weight"] = torch.zeros((N, N), dtype=torch.uint8)
+        for s in ("_mx", "_rx", "_my", "_ry"):
+            m.w[att + n + ".weight" + s] = torch.zeros(N, dtype=torch.float16)
+    monkeypatch.setattr(ops, "mm8_seq_batch", lambda *a: True)
+    x, sx = torch.zeros((3, N), dtype=torch.float16), torch.zeros((3, N), dtype=torch.float16)
+    f32 = [torch.zeros(3, N) for _ in range(3)]
+    m._att_seq_v4(x, [sx] + f32 + [sx], 0, rows=True)
+    for i in range(3):
+        bad = list(f32)
+        bad[i] = bad[i].half()
+        with pytest.raises(_lib.RwkvB200Error, match="fp32"):
+            m._att_seq_v4(x, [sx] + bad + [sx], 0, rows=True)
