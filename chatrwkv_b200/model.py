@@ -1018,6 +1018,7 @@ class RWKV:
         library throughout; the four small low-rank products of RWKV-6 (ranks 32..160) are plain fp16 library GEMMs
         as in the reference (`@`, `bmm`)."""
         import ctypes as C
+        ops._require(st2[1].dtype == torch.float32, "the wkv state must be fp32")
         w, a, L = self.w, self.args, lib()
         T, D = x.shape
         H = a.n_head

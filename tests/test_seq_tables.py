@@ -97,3 +97,11 @@ def test_batched_rwkv4_step_refuses_states_that_are_not_fp32(monkeypatch):
         bad[i] = bad[i].half()
         with pytest.raises(_lib.RwkvB200Error, match="fp32"):
             m._att_seq_v4(x, [sx] + bad + [sx], 0, rows=True)
+
+
+@pytest.mark.parametrize("rows", [False, True])
+def test_rwkv56_states_that_are_not_fp32_are_refused(rows):
+    m = RWKV.__new__(RWKV)
+    x, sx = torch.zeros((3, N), dtype=torch.float16), torch.zeros(N, dtype=torch.float16)
+    with pytest.raises(_lib.RwkvB200Error, match="fp32"):
+        m._att_seq_v56(x, [sx, torch.zeros((2, 16, 16), dtype=torch.float16)], 0, rows=rows)
