@@ -1250,25 +1250,10 @@ class RWKV:
         return self._mm_epi(xln, "head.weight", EPI_STORE, early=early)
 
     def _stage_tokens(self, tokens):
-        """Token ids to the device through pinned memory (two slots, reused in turn): a copy from pageable memory would
-        make the host wait for everything queued before it, so consecutive chunks of a prompt could not be queued ahead."""
-        T = len(tokens)
-        if not hasattr(self, "_seq_tok"):
-            self._seq_tok = [None, None]
-            self._seq_tok_ev = [None, None]
-            self._seq_tok_slot = 0
-        slot = self._seq_tok_slot = 1 - self._seq_tok_slot
-        if self._seq_tok_ev[slot] is not None:
-            self._seq_tok_ev[slot].synchronize()
-        if self._seq_tok[slot] is None or self._seq_tok[slot].numel() < T:
-            self._seq_tok[slot] = torch.empty(max(4096, T), dtype=torch.int64).pin_memory()
-            self._seq_tok_ev[slot] = torch.cuda.Event()
-        host = self._seq_tok[slot][:T]
-        host.copy_(torch.tensor(tokens, dtype=torch.int64))
-        idx = torch.empty(T, dtype=torch.int64, device=self.device)
-        idx.copy_(host, non_blocking=True)
-        self._seq_tok_ev[slot].record(torch.cuda.current_stream(self.device))
-        return idx
+        """Token ids to the device through pinned memory: a copy from pageable memory would make the host wait for everything
+        queued before it, so consecutive chunks of a prompt could not be queued ahead.  The buffer is torch's pinned pool's,
+        which hands it out again only when the copy is over (calls of several threads never share one)."""
+        return torch.tensor(tokens, dtype=torch.int64, pin_memory=True).to(self.device, non_blocking=True)
 
     # The group norm of RWKV-5/6 divides by nearly nothing at the first positions of an empty state: there two correct
     # summation orders of the same matmul end up percents apart, and the difference fades as 1 / T (state entries: 0.4 of
