@@ -248,11 +248,13 @@ __global__ void __launch_bounds__(kT) lora_b_kernel(const LoraB b) {
 }
 
 // One-step WKV of RWKV-5.2 / RWKV-6 for one token, then group-norm (eps 64e-5) and the gate.
-// State in the model's layout [H, key j, value i] (pkg/model.py:1461-1471).  grid = heads of all sequences, block = 256;
-// u and ln_x (and w unless every sequence has its own) are those of head % Hp.  Bound by the state's 32 KB per head of 64
-// once many sequences run at once (64 x 64 heads: 134 MB in and out):
+// State in the model's layout [H, key j, value i] (pkg/model.py:1461-1471).  grid = (heads, sequences), block = 256; u and
+// ln_x (and w unless every sequence has its own) are per head.  Bound by the state's 32 KB per head of 64 once many sequences
+// run at once (64 x 64 heads: 134 MB in and out); one sequence (ROWS false) is a chain of latencies, kept free of the
+// sequences' address arithmetic.
 // thread (q, i) covers the keys j = q, q + TPI, ... of value index i (TPI = 256 / N threads per i).
-__global__ void __launch_bounds__(kT) wkv56_one_kernel(int N, int Hp, int w_per_row, const __half* __restrict__ r, const __half* __restrict__ k,
+template <bool ROWS>
+__global__ void __launch_bounds__(kT) wkv56_one_kernel(int N, int w_per_row, const __half* __restrict__ r, const __half* __restrict__ k,
                                                       const __half* __restrict__ v, const float* __restrict__ w,
                                                       const float* __restrict__ u, const float* s_in, float* s_out,
                                                       const float* __restrict__ lnx_w, const float* __restrict__ lnx_b,
@@ -260,19 +262,19 @@ __global__ void __launch_bounds__(kT) wkv56_one_kernel(int N, int Hp, int w_per_
     extern __shared__ float sm[];               // rr[N] kk[N] ww[N] uu[N] | acc[TPI][N]
     __shared__ float sh8[kT / 32];
     float* rr = sm; float* kk = sm + N; float* ww = sm + 2 * N; float* uu = sm + 3 * N; float* accs = sm + 4 * N;
-    const int hh = blockIdx.x, tid = threadIdx.x;
-    const long long c0 = (long long)hh * N;
-    const int p0 = (hh % Hp) * N;
+    const int tid = threadIdx.x, p0 = blockIdx.x * N;
+    const long long row = ROWS ? (long long)blockIdx.y * gridDim.x : 0;       // heads before this sequence's
+    const long long c0 = row * N + p0, s0 = (row + blockIdx.x) * N * N;
     pdl_open();
     {   // the head's state (written a token ago)
-        const char* base = reinterpret_cast<const char*>(s_in + (long long)hh * N * N);
+        const char* base = reinterpret_cast<const char*>(s_in + s0);
         for (long long o = (long long)tid * 128; o < (long long)N * N * 4; o += (long long)kT * 128) l2_line(base + o);
     }
     pdl_wait();
     for (int j = tid; j < N; j += kT) {
         rr[j] = __half2float(__ldcg(r + c0 + j));
         kk[j] = __half2float(__ldcg(k + c0 + j));
-        ww[j] = __ldcg(w + (w_per_row ? c0 : (long long)p0) + j);
+        ww[j] = __ldcg(w + (ROWS && w_per_row ? c0 : p0) + j);
         uu[j] = u[p0 + j];
     }
     __syncthreads();
@@ -281,8 +283,8 @@ __global__ void __launch_bounds__(kT) wkv56_one_kernel(int N, int Hp, int w_per_
     float acc = 0.f;
     if (q < TPI && tid < TPI * N) {
         const float vi = __half2float(__ldcg(v + c0 + i));
-        const float* si = s_in + (long long)hh * N * N + i;
-        float* so = s_out + (long long)hh * N * N + i;
+        const float* si = s_in + s0 + i;
+        float* so = s_out + s0 + i;
         for (int jb = q; jb < N; jb += 16 * TPI) {      // 16 state values in flight, then the updates
             float sv[16];
 #pragma unroll
@@ -741,10 +743,20 @@ extern "C" int rwkv_wkv56_one_rows(int64_t B, int64_t H, int64_t N, const void* 
     RWKV_CHECK_ARG(B >= 1 && H >= 1 && N >= 1 && N <= kT && B * H <= INT32_MAX);
     RWKV_CHECK_ARG(r && k && v && w && u && state && new_state && lnx_w && lnx_b && g && out);
     const int TPI = kT / int(N) > 0 ? kT / int(N) : 1;
-    return rwkv_launch_pdl(wkv56_one_kernel, dim3(unsigned(B * H)), dim3(kT), (4 * N + TPI * N) * sizeof(float),
-                           static_cast<cudaStream_t>(stream), int(N), int(H), w_per_row, static_cast<const __half*>(r),
-                           static_cast<const __half*>(k), static_cast<const __half*>(v), w, u, state, new_state, lnx_w, lnx_b,
-                           static_cast<const __half*>(g), static_cast<__half*>(out));
+    const size_t smem = (4 * N + TPI * N) * sizeof(float);
+    auto launch = [&](auto kernel, int64_t first, int64_t rows) {
+        const int64_t c = first * H * N, s = c * N;
+        return rwkv_launch_pdl(kernel, dim3(unsigned(H), unsigned(rows)), dim3(kT), smem, static_cast<cudaStream_t>(stream), int(N),
+                               w_per_row, static_cast<const __half*>(r) + c, static_cast<const __half*>(k) + c,
+                               static_cast<const __half*>(v) + c, w + (w_per_row ? c : 0), u, state + s, new_state + s, lnx_w, lnx_b,
+                               static_cast<const __half*>(g) + c, static_cast<__half*>(out) + c);
+    };
+    if (B == 1) return launch(wkv56_one_kernel<false>, 0, 1);
+    for (int64_t b = 0; b < B; b += 65535) {               // the grid's limit along y
+        const int rc = launch(wkv56_one_kernel<true>, b, B - b < 65535 ? B - b : 65535);
+        if (rc != RWKV_OK) return rc;
+    }
+    return RWKV_OK;
 }
 
 // Token shift + decay of one RWKV-6 layer in one single-cluster launch (see v6_att_pre_kernel).
