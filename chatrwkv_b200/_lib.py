@@ -14,7 +14,7 @@ LIB_PATH = os.path.join(_HERE, "librwkv_b200.so")
 OK = 0
 F32, F16, BF16 = 0, 1, 2
 PRO_PLAIN, PRO_LN_MIX, PRO_WKV4, PRO_GN_GATE = 0, 1, 2, 3
-ERR_UNSUPPORTED = -5
+ERR_WORKSPACE, ERR_UNSUPPORTED = -3, -5
 MM8_WIDE_BUILD = 1
 SEQ_F16_SUMS = 0x100      # added to an epilogue of mm8_seq_epi
 EPI_ACC_F32, EPI_STORE, EPI_SIGMOID, EPI_RELU_SQ, EPI_RESIDUAL, EPI_MUL_RESIDUAL, EPI_STORE_F32, EPI_SILU = range(8)

@@ -889,18 +889,17 @@ class RWKV:
         y = out if out is not None else torch.empty((x.shape[0], M), dtype=torch.float16, device=x.device)
         return ops.mm8_seq_epi(x, wq, mx, rx, my, ry, y, epilogue, aux, aux2, out_scale)
 
-    def _seq_group(self, kind, jobs, mode=0, ln=None, mixes=None):
-        """The table of a launch of 1..4 int8 matrices (rwkv_mm8_seq_batch) with what the model fixes, and its length:
-        `jobs` = [(name, epilogue)], `ln` = the names of the norm's weight and bias, `mixes` = names.  The matrices' part is
-        made once (`_scales` keeps their tensors); every call gets a copy of its own, in which it sets the activations'
-        addresses (calls of several threads may be filling theirs at the same time), with the norm and the mixes as `self.w`
-        has them now.  (None, 0) when a matrix is kept in fp16 or split over ranks."""
+    def _seq_group(self, kind, jobs, mode=0):
+        """A table for a launch of 1..4 int8 matrices (rwkv_mm8_seq_batch), `jobs` = [(name, epilogue)], with the matrices
+        filled in, and their out-feature counts.  The matrices' part is made once (`_scales` keeps their tensors); every call
+        gets a copy of its own, in which the caller sets the addresses of norms, mixes and activations (calls of several threads
+        may be filling theirs at the same time).  (None, None) when a matrix is kept in fp16 or split over ranks."""
         key = jobs[0][0], kind
         t = self._seq_tables.get(key)
         if t is None:
             w = self.w
             if self._world > 1 or any(w[name].dtype != torch.uint8 for name, _ in jobs):
-                t = self._seq_tables[key] = (None, 0)
+                t = self._seq_tables[key] = (None, None)
                 return t
             arr = (_lib.Mm8SeqProblem * len(jobs))()
             for i, (name, epi) in enumerate(jobs):
@@ -909,34 +908,35 @@ class RWKV:
                 q.w, q.w_stride, q.M = wq.data_ptr(), wq.stride(0), wq.shape[1]
                 q.mx, q.rx, q.my, q.ry = mx.data_ptr(), rx.data_ptr(), my.data_ptr(), ry.data_ptr()
                 q.epilogue, q.out_scale, q.kind, q.mode = epi, 1.0, kind, mode
-            t = self._seq_tables[key] = (arr, len(jobs))
-        const, n = t
-        if not n:
-            return t
-        arr = type(const).from_buffer_copy(const)
-        if ln is not None:
-            arr[0].ln_w, arr[0].ln_b = self.w[ln[0]].data_ptr(), self.w[ln[1]].data_ptr()
-        if mixes is not None:
-            for q, name in zip(arr, mixes):
-                q.mix = self.w[name].data_ptr()
-        return arr, n
+            t = self._seq_tables[key] = (arr, [q.M for q in arr])
+        const, Ms = t
+        return (t if const is None else (type(const).from_buffer_copy(const), Ms))
 
     def _ln_mix_group(self, x, sx, rows, jobs, mode, ln, mixes):
-        """LayerNorm, token shift and the matmuls of the mixes as two launches (operands, matmuls).  Returns the outputs and
-        the new shift state, or None where the separate launches have to run."""
+        """LayerNorm, token shift and the matmuls of the mixes as two launches (operands, matmuls).  `ln`: the names of the
+        norm's weight and bias, `mixes`: names.  Returns the outputs and the new shift state, or None where the separate
+        launches have to run."""
         T, D = x.shape
-        arr, n = self._seq_group(PRO_LN_MIX, jobs, mode, ln, mixes)
+        arr, Ms = self._seq_group(PRO_LN_MIX, jobs, mode)
         if arr is None:
             return None
-        outs = [torch.empty((T, q.M), dtype=torch.float16, device=x.device) for q in arr]
+        w, dev = self.w, x.device
+        xp, xs = x.data_ptr(), x.stride(0)
+        outs = [torch.empty((T, M), dtype=torch.float16, device=dev) for M in Ms]
         new_sx = torch.empty_like(sx) if sx is not None else None
-        for q, y in zip(arr, outs):
-            q.x, q.x_stride, q.y, q.y_stride = x.data_ptr(), x.stride(0), y.data_ptr(), y.stride(0)
-        if sx is not None:
-            q = arr[0]
-            q.sx, q.sx_stride = sx.data_ptr(), (sx.stride(0) if rows else 0)
-            q.xx_out, q.xx_stride, q.new_state = (new_sx.data_ptr(), new_sx.stride(0), None) if rows else (None, 0, new_sx.data_ptr())
-        if not ops.mm8_seq_batch(arr, n, T, D, x.device):
+        for i, (q, y) in enumerate(zip(arr, outs)):
+            q.x, q.x_stride, q.y, q.y_stride = xp, xs, y.data_ptr(), Ms[i]
+            if mixes is not None:
+                q.mix = w[mixes[i]].data_ptr()
+            if i == 0:
+                q.ln_w, q.ln_b = w[ln[0]].data_ptr(), w[ln[1]].data_ptr()
+                if sx is not None:
+                    q.sx, q.sx_stride = sx.data_ptr(), (sx.stride(0) if rows else 0)
+                    if rows:
+                        q.xx_out, q.xx_stride = new_sx.data_ptr(), new_sx.stride(0)
+                    else:
+                        q.new_state = new_sx.data_ptr()
+        if not ops.mm8_seq_batch(arr, len(Ms), T, D, dev):
             return None
         return outs, new_sx
 
@@ -1065,12 +1065,12 @@ class RWKV:
                     (att + "gate.weight", EPI_SILU)]
 
             def matmuls():      # fp16-rounded r, k, v: the kernel widens them (model.py:1413, 1425-1427)
-                arr, n = self._seq_group(PRO_PLAIN, jobs)
+                arr, Ms = self._seq_group(PRO_PLAIN, jobs)
                 if arr is not None and not early:
-                    outs = [torch.empty((T, q.M), dtype=torch.float16, device=dev) for q in arr]
+                    outs = [torch.empty((T, M), dtype=torch.float16, device=dev) for M in Ms]
                     for q, xm, ym in zip(arr, (rx, kx, vx, gx), outs):
                         q.x, q.x_stride, q.y, q.y_stride = xm.data_ptr(), xm.stride(0), ym.data_ptr(), ym.stride(0)
-                    if ops.mm8_seq_batch(arr, n, T, D, dev):
+                    if ops.mm8_seq_batch(arr, len(Ms), T, D, dev):
                         return outs
                 return [self._mm_epi(xm, name, epi, early=early) for xm, (name, epi) in zip((rx, kx, vx, gx), jobs)]
             if rows:
@@ -1109,9 +1109,10 @@ class RWKV:
             return self._mm_epi(out, att + "output.weight", EPI_RESIDUAL, aux=x, out=x)
         y = torch.empty((T, D), dtype=torch.float32, device=dev)
         ops.wkv56_seq(self.version == 6, H, S_in, r, k, v, decay, u, y, model_layout=True, state_out=S)
-        arr, _ = self._seq_group(PRO_GN_GATE, [(att + "output.weight", EPI_RESIDUAL)], ln=(att + "ln_x.weight", att + "ln_x.bias"))
+        arr, _ = self._seq_group(PRO_GN_GATE, [(att + "output.weight", EPI_RESIDUAL)])
         if arr is not None and not early:
             q = arr[0]
+            q.ln_w, q.ln_b = w[att + "ln_x.weight"].data_ptr(), w[att + "ln_x.bias"].data_ptr()
             q.x, q.x_stride, q.gate, q.gate_stride, q.head, q.eps = y.data_ptr(), D, g.data_ptr(), g.stride(0), N, 64e-5
             q.y, q.y_stride, q.aux, q.aux_stride = x.data_ptr(), x.stride(0), x.data_ptr(), x.stride(0)
             if ops.mm8_seq_batch(arr, 1, T, D, dev):

@@ -165,11 +165,15 @@ def mm8_seq_epi(x, w, mx, rx, my, ry, y, epilogue, aux=None, aux2=None, out_scal
 def mm8_seq_batch(problems, n, B, N, device):
     """1..4 matrices on B rows in one launch (`problems`: an array of `_lib.Mm8SeqProblem`; rwkv_mm8_seq_batch in the
     header).  False where the tensor-core kernel does not take the operands: nothing has been launched then."""
-    nbytes = lib().rwkv_mm8_seq_batch_workspace_bytes(problems, n, B, N)
-    if nbytes == 0:
-        return False
-    ws = workspace(device, nbytes, "mm8_seq")
-    rc = lib().rwkv_mm8_seq_batch(problems, n, B, N, ws.data_ptr(), ws.numel(), _stream(device))
+    st = _stream(device)
+    ws = _workspaces.get(("mm8_seq", device.index, st))
+    rc = _lib.ERR_WORKSPACE if ws is None else lib().rwkv_mm8_seq_batch(problems, n, B, N, ws.data_ptr(), ws.numel(), st)
+    if rc == _lib.ERR_WORKSPACE:        # none yet, or too small for this launch: nothing has been launched
+        nbytes = lib().rwkv_mm8_seq_batch_workspace_bytes(problems, n, B, N)
+        if nbytes == 0:
+            return False
+        ws = workspace(device, nbytes, "mm8_seq")
+        rc = lib().rwkv_mm8_seq_batch(problems, n, B, N, ws.data_ptr(), ws.numel(), st)
     if rc == _lib.ERR_UNSUPPORTED:
         return False
     check(rc, "mm8_seq_batch")
