@@ -6,12 +6,15 @@
 // with x' = x*ry, SX = sum_k x, SXR = sum_k x', SXMY = sum_k x*my (per row t), the factorisation of mm8_one.
 //   * x' becomes a 24-bit fixed-point integer per row (the scale is the power of two that takes the row's largest
 //     magnitude into [2^22, 2^23), so the fp32 products are scaled exactly and rounded once, to 2^-23 .. 2^-22 of the
-//     row's maximum) and enters as three planes of signed base-256 digits;
+//     row's maximum) and enters as three planes of signed base-256 digits.  A row in which a few elements tower over the
+//     rest (outlier channels) is WIDE: it gets 32 bits, the last 8 as a fourth plane, for which a token tile that holds
+//     such a row takes its K range a second time;
 //   * W enters as the raw uint8 rows: TMA brings 128-column x 128-row boxes into shared memory in the layout the
 //     tensor core reads as a transposed (MN-major) operand, with no conversion and no thread touching a weight;
 //   * all sums are exact 32-bit integers (128 * 255 * K < 2^31 up to K = 65536), the planes and the K splits are
-//     combined in exact 64-bit integers and rounded to fp32 once: results do not depend on the tiling, on the split or
-//     on the form of the kernel.
+//     combined in exact 64-bit integers and rounded to fp32 once: the product part does not depend on the tiling, on the
+//     split, on the form of the kernel or on the other rows.  (SX, SXR and SXMY are fp32 sums of the operand pass, whose
+//     order depends on the launch's rows and on N.)
 // W's 128 columns are the M side of the MMA and the tokens of all three planes its N side, so a launch of 16 tokens
 // multiplies 48 columns instead of padding 16 rows to 128.
 //
@@ -31,6 +34,7 @@
 #include "common.cuh"
 #include "seq_epi.cuh"
 #include <algorithm>
+#include <cmath>
 #include <cuda.h>
 #include "mm8_seq_i8.h"
 
@@ -48,7 +52,7 @@ constexpr int kSmemBudget = 226 * 1024;
 constexpr unsigned kWaitLimitI8 = 1u << 22;
 constexpr float kTopDigits = 8355711.f;         // 127 * 65536 + 127 * 256 + 127
 
-struct alignas(16) RowConst { float scale, sx, sxr, sxmy; long long corr, pad; };      // corr = -128 * sum of the integers
+struct alignas(16) RowConst { float scale, sx, sxr, sxmy; long long corr; int wide, pad; };     // corr = -128 * sum of the integers
 
 struct I8Problem {
     const __half* mx; const __half* rx;
@@ -60,6 +64,7 @@ struct I8Problem {
 struct alignas(64) I8Args {
     CUtensorMap wmap[kSeqI8MaxProblems];
     CUtensorMap xmap[2];                        // the token planes as rows of 128 bytes, in boxes of the rows of each MMA
+    CUtensorMap lmap;                           // the fourth planes
     I8Problem p[kSeqI8MaxProblems];
     const RowConst* consts;                     // [problem][T]
     unsigned* tickets;                          // [split tile][CTA of the pair]
@@ -163,7 +168,8 @@ template <int PAIR> __device__ __forceinline__ void commit_i8(uint32_t bar) {
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
     }
 }
-// fp32 of an exact 64-bit sum below 2^54, rounded once
+// fp32 of an exact 64-bit sum.  Three digits (below 2^47 up to K = 65536): both parts are exact, rounded once.  Four digits
+// (below 2^54): above 2^48 the upper part is rounded to 24 bits before, which makes it one unit in the last place.
 __device__ __forceinline__ float sum_to_f32(long long s) {
     return fmaf((float)(int)(s >> 24), 16777216.f, (float)((int)s & 0xffffff));
 }
@@ -181,6 +187,12 @@ __device__ __forceinline__ void epi8(int mode, float scale, const __half (&v)[8]
     }
 }
 __device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory"); }
+__device__ __forceinline__ bool epi_sync_or(bool v) {                    // the same, with the OR of `v` over its threads
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(r) : "r"((uint32_t)v), "n"(kEpiThreads) : "memory");
+    return r != 0;
+}
 __device__ __forceinline__ void tmem_ld8(int (&v)[8], uint32_t addr) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
@@ -273,14 +285,15 @@ struct PrepProblem {
 struct PrepArgs {
     PrepProblem p[kSeqI8MaxProblems];
     int nprob, T, N, nkb, TT, ntt, ntickets, vec;          // vec: every vector and row starts on a 16-byte boundary
-    uint8_t* images; RowConst* consts; unsigned* tickets;
+    float narrow;                                // a row whose squared norm, in integer units of three digits, is below this is wide
+    uint8_t* images; uint8_t* low; RowConst* consts; unsigned* tickets;
 };
-// Sums (MAX0: the first value's maximum) of NV values per thread over the block; every thread gets the results.
-template <int NV, bool MAX0>
+// Sums of NV values per thread over the block; every thread gets the results.
+template <int NV>
 __device__ __forceinline__ void block_reduce(float (&v)[NV], float (*sh)[32]) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) v[i] = (MAX0 && i == 0) ? warp_max(v[i]) : warp_sum(v[i]);
+    for (int i = 0; i < NV; ++i) v[i] = warp_sum(v[i]);
     __syncthreads();                                       // the previous use of sh is over
     if (lane == 0) {
 #pragma unroll
@@ -288,10 +301,33 @@ __device__ __forceinline__ void block_reduce(float (&v)[NV], float (*sh)[32]) {
     }
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-        const float t = lane < nwarp ? sh[i][lane] : 0.f;      // (maxima are of magnitudes)
-        v[i] = (MAX0 && i == 0) ? warp_max(t) : warp_sum(t);
-    }
+    for (int i = 0; i < NV; ++i) v[i] = warp_sum(lane < nwarp ? sh[i][lane] : 0.f);
+}
+// The row's maximum (of magnitudes: their bits order like integers) and four sums over the block, for every thread.  The sums
+// run the butterfly of warp_sum with half of the values dropped at each step while there are several: the same pairs in the
+// same order in 6 shuffles instead of 20, and again over the warps' parts.
+__device__ __forceinline__ void row_reduce(float (&v)[5], float (*sh)[32]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+    const bool b4 = (lane & 16) != 0, b3 = (lane & 8) != 0;
+    auto fold = [&](float s0, float s1, float s2, float s3) {         // lanes 8 i .. 8 i + 7 get sum i
+        float x = (b4 ? s2 : s0) + __shfl_xor_sync(0xffffffffu, b4 ? s0 : s2, 16);
+        const float y = (b4 ? s3 : s1) + __shfl_xor_sync(0xffffffffu, b4 ? s1 : s3, 16);
+        x = (b3 ? y : x) + __shfl_xor_sync(0xffffffffu, b3 ? x : y, 8);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        return x;
+    };
+    const float m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v[0])));
+    const float s = fold(v[1], v[2], v[3], v[4]);
+    __syncthreads();                                       // the previous use of sh is over
+    if (lane == 0) sh[0][warp] = m;
+    if ((lane & 7) == 0) sh[1 + (lane >> 3)][warp] = s;
+    __syncthreads();
+    const bool part = lane < nwarp;
+    v[0] = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(part ? sh[0][lane] : 0.f)));
+    const float t = fold(part ? sh[1][lane] : 0.f, part ? sh[2][lane] : 0.f, part ? sh[3][lane] : 0.f, part ? sh[4][lane] : 0.f);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[1 + i] = __shfl_sync(0xffffffffu, t, 8 * i);
 }
 
 // PRO: where the rows of x come from (RWKV_PRO_*).  LOOP (RWKV_PRO_PLAIN only): a thread owns every blockDim-th E k and
@@ -301,7 +337,7 @@ template <int PRO, int E, bool LOOP, bool PRE, int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB) mm8_seq_i8_prep(const __grid_constant__ PrepArgs a) {
     asm volatile("griddepcontrol.launch_dependents;");
     const int t = blockIdx.x, tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarp = nthr >> 5;
-    __shared__ float sh[4][32];
+    __shared__ float sh[5][32];
     __shared__ long long shq[32];
     const bool vec = a.vec != 0;
     const int N = a.N, k0 = tid * E;
@@ -339,7 +375,7 @@ __global__ void __launch_bounds__(MAXT, MINB) mm8_seq_i8_prep(const __grid_const
         float m[2] = {0.f, 0.f}, d[2] = {0.f, 0.f};
 #pragma unroll
         for (int e = 0; e < E; ++e) { m[0] += xx[e]; m[1] += prev[e]; }
-        block_reduce<2, false>(m, sh);
+        block_reduce<2>(m, sh);
         m[0] /= float(N); m[1] /= float(N);
 #pragma unroll
         for (int e = 0; e < E; ++e)
@@ -347,7 +383,7 @@ __global__ void __launch_bounds__(MAXT, MINB) mm8_seq_i8_prep(const __grid_const
                 d[0] = fmaf(xx[e] - m[0], xx[e] - m[0], d[0]);
                 d[1] = fmaf(prev[e] - m[1], prev[e] - m[1], d[1]);
             }
-        block_reduce<2, false>(d, sh);
+        block_reduce<2>(d, sh);
         const float r0 = rsqrtf(d[0] / float(N) + 1e-5f), r1 = rsqrtf(d[1] / float(N) + 1e-5f);
 #pragma unroll
         for (int e = 0; e < E; e += 2) {
@@ -417,7 +453,7 @@ __global__ void __launch_bounds__(MAXT, MINB) mm8_seq_i8_prep(const __grid_const
         const bool have = PRE && prob == (int)blockIdx.y;  // the vectors are in registers
         const __half* xrow = static_cast<const __half*>(p.x) + (long long)t * p.x_stride;      // RWKV_PRO_PLAIN
         HV<E> xv = zero_hv<E>();
-        float red[4] = {0.f, 0.f, 0.f, 0.f};               // maximum, SX, SXR, SXMY
+        float red[5] = {0.f, 0.f, 0.f, 0.f, 0.f};          // maximum, SX, SXR, SXMY, sum of squares of x'
         auto first = [&](int c) {
             const int kc = c * E;
             if constexpr (PRO == RWKV_PRO_PLAIN) {
@@ -444,43 +480,52 @@ __global__ void __launch_bounds__(MAXT, MINB) mm8_seq_i8_prep(const __grid_const
                 red[1] += xe;
                 red[2] += xp;
                 red[3] = fmaf(xe, my[e], red[3]);
+                red[4] = fmaf(xp, xp, red[4]);
                 red[0] = fabsf(xp) <= 3.0e38f ? fmaxf(red[0], fabsf(xp)) : INFINITY;      // fmaxf would drop a NaN
             }
         };
         if constexpr (!LOOP) { if (mine) first(tid); }
         else for (int c = tid; c < nchunk; c += nthr) first(c);
-        block_reduce<4, true>(red, sh);
+        row_reduce(red, sh);
         // the power of two `up` that takes the maximum into [2^22, 2^23), or half of it if three digits would not hold it
         float up = 0.f, down = 0.f;
+        bool wide = false;
         if (red[0] > 0.f && red[0] <= 3.0e38f) {
             int e = 22 - ilogbf(red[0]);
             if (ldexpf(red[0], e) > kTopDigits) --e;
             up = ldexpf(1.f, e);                            // |x'| >= 2^-48 or 0: e <= 70
-            down = ldexpf(1.f, -e);
+            wide = red[4] * up * up < a.narrow;             // (see wide_norm)
+            down = ldexpf(1.f, wide ? -e - 8 : -e);
         } else if (red[0] > 0.f) {
             down = NAN;                                     // a NaN or an infinity among the activations: the row is NaN
         }
         uint8_t* img = a.images + ((size_t)prob * a.ntt + tt) * a.nkb * (size_t)(3 * a.TT * BKI) + (size_t)ti * BKI;
+        // balanced base-256 digits of four neighbouring k: the bytes of q + 128 * (1 + 256 + 65536), each minus 128
+        auto digits = [&](const int (&q)[4], uint32_t& d0, uint32_t& d1, uint32_t& d2) {
+            uint32_t u[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) u[i] = (uint32_t)(q[i] + 0x808080);
+            const uint32_t lo01 = __byte_perm(u[0], u[1], 0x5140), lo23 = __byte_perm(u[2], u[3], 0x5140);
+            const uint32_t hi01 = __byte_perm(u[0], u[1], 0x0062), hi23 = __byte_perm(u[2], u[3], 0x0062);
+            d0 = __byte_perm(lo01, lo23, 0x5410) ^ 0x80808080u;
+            d1 = __byte_perm(lo01, lo23, 0x7632) ^ 0x80808080u;
+            d2 = __byte_perm(hi01, hi23, 0x5410) ^ 0x80808080u;
+        };
+        auto in_row = [&](int kc) { return (size_t)((((kc >> 4) & 7) ^ (ti & 7)) << 4) + (kc & 15); };
         auto second = [&](int c, int& isum) {
-            // balanced base-256 digits: the bytes of q + 128 * (1 + 256 + 65536), each minus 128
             uint32_t d[3][E / 4];
 #pragma unroll
             for (int e = 0; e < E; e += 4) {
-                uint32_t u[4];
+                int q[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const int q = up > 0.f ? __float2int_rn(xv[e + i] * ry[e + i] * up) : 0;
-                    isum += q;
-                    u[i] = (uint32_t)(q + 0x808080);
+                    q[i] = up > 0.f ? __float2int_rn(xv[e + i] * ry[e + i] * up) : 0;
+                    isum += q[i];
                 }
-                const uint32_t lo01 = __byte_perm(u[0], u[1], 0x5140), lo23 = __byte_perm(u[2], u[3], 0x5140);
-                const uint32_t hi01 = __byte_perm(u[0], u[1], 0x0062), hi23 = __byte_perm(u[2], u[3], 0x0062);
-                d[0][e >> 2] = __byte_perm(lo01, lo23, 0x5410) ^ 0x80808080u;
-                d[1][e >> 2] = __byte_perm(lo01, lo23, 0x7632) ^ 0x80808080u;
-                d[2][e >> 2] = __byte_perm(hi01, hi23, 0x5410) ^ 0x80808080u;
+                digits(q, d[0][e >> 2], d[1][e >> 2], d[2][e >> 2]);
             }
             const int kc = c * E;
-            uint8_t* dst = img + (size_t)(kc >> 7) * (3 * plane) + ((((kc >> 4) & 7) ^ (ti & 7)) << 4) + (kc & 15);
+            uint8_t* dst = img + (size_t)(kc >> 7) * (3 * plane) + in_row(kc);
             typedef typename VecOf<E>::T V;
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
@@ -489,8 +534,41 @@ __global__ void __launch_bounds__(MAXT, MINB) mm8_seq_i8_prep(const __grid_const
                 *reinterpret_cast<V*>(dst + i * plane) = o;
             }
         };
+        // a wide row: 32 bits, the first 24 as above and the last digit to the fourth plane (rare: kept small, four k at a time)
+        auto second_wide = [&](int c) -> long long {
+            const int kc = c * E;
+            uint8_t* dst = img + (size_t)(kc >> 7) * (3 * plane) + in_row(kc);
+            uint8_t* low = a.low + (((size_t)prob * a.ntt + tt) * a.nkb + (kc >> 7)) * plane + (size_t)ti * BKI + in_row(kc);
+            const float up4 = up * 256.f;
+            int isum = 0, lsum = 0;
+#pragma unroll
+            for (int e = 0; e < E; e += 4) {
+                int q[4], l[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    q[i] = __float2int_rn(xv[e + i] * ry[e + i] * up4);
+                    l[i] = (int8_t)q[i];
+                    q[i] = (q[i] + 128) >> 8;               // (q - l) / 256
+                    isum += q[i];
+                    lsum += l[i];
+                }
+                uint32_t d[3];
+                digits(q, d[0], d[1], d[2]);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(dst + i * plane + e) = d[i];
+                *reinterpret_cast<uint32_t*>(low + e) = __byte_perm(__byte_perm(l[0], l[1], 0x0040), __byte_perm(l[2], l[3], 0x0040), 0x5410);
+            }
+            return 256ll * isum + lsum;
+        };
         long long qsum = 0;
-        if constexpr (!LOOP) {
+        if (__builtin_expect(wide, 0)) {
+            if constexpr (!LOOP) { if (mine) qsum = second_wide(tid); }
+            else for (int c = tid; c < nchunk; c += nthr) {
+                xv = load_hv<E>(xrow, c * E, N, vec);
+                ry = load_hv<E, true>(p.ry, c * E, N, vec);
+                qsum += second_wide(c);
+            }
+        } else if constexpr (!LOOP) {
             int isum = 0;
             if (mine) second(tid, isum);
             qsum = isum;
@@ -514,7 +592,8 @@ __global__ void __launch_bounds__(MAXT, MINB) mm8_seq_i8_prep(const __grid_const
             for (int o = 16; o > 0; o >>= 1) qsum += __shfl_xor_sync(0xffffffffu, qsum, o);
             if (lane == 0) {
                 RowConst rc;
-                rc.scale = down; rc.sx = red[1]; rc.sxr = red[2]; rc.sxmy = red[3]; rc.corr = -128 * qsum; rc.pad = 0;
+                rc.scale = down; rc.sx = red[1]; rc.sxmy = red[3]; rc.corr = -128 * qsum; rc.wide = wide ? 1 : 0; rc.pad = 0;
+                rc.sxr = wide ? __ll2float_rn(qsum) * down : red[2];       // wide: the exact sum of the integers
                 a.consts[(size_t)prob * a.T + t] = rc;
             }
         }
@@ -546,6 +625,24 @@ template <int PAIR> __device__ __forceinline__ bool item_of(const I8Args& a, int
     return true;
 }
 
+// Whether a token tile holds a wide row, in two steps so that the loads (of one warp) run beside other work.  The same
+// answer in every role and in both CTAs of a pair.
+struct WideFlags { int v[kMaxTT / 32]; };
+__device__ __forceinline__ WideFlags wide_flags(const I8Args& a, const Item& tl, int lane) {
+    WideFlags f;
+    const int t0 = tl.tt * a.TT, n = min(a.TT, a.T - t0);
+    const RowConst* rc = a.consts + (size_t)tl.prob * a.T + t0;
+#pragma unroll
+    for (int i = 0; i < kMaxTT / 32; ++i) f.v[i] = lane + 32 * i < n ? __ldcg(&rc[lane + 32 * i].wide) : 0;
+    return f;
+}
+__device__ __forceinline__ bool any_wide(const WideFlags& f) {
+    int v = 0;
+#pragma unroll
+    for (int i = 0; i < kMaxTT / 32; ++i) v |= f.v[i];
+    return __any_sync(0xffffffffu, v != 0);
+}
+
 template <int PAIR>
 __global__ void __launch_bounds__(kThreadsI8, 1) mm8_seq_i8_kernel(const __grid_constant__ I8Args a) {
     asm volatile("griddepcontrol.launch_dependents;");
@@ -557,6 +654,7 @@ __global__ void __launch_bounds__(kThreadsI8, 1) mm8_seq_i8_kernel(const __grid_
     const int S = a.stages;
     const int n1 = a.N1 / PAIR, n2 = a.N2 / PAIR;                 // token rows of each MMA that this CTA holds
     const uint32_t xbytes = (uint32_t)(n1 + n2) * BKI, stage_bytes = kWTile + xbytes;
+    const int n3 = a.TT / PAIR;                                   // of the fourth plane
     uint8_t* bars = smem + (size_t)S * stage_bytes;
     const uint32_t full0 = su(bars), empty0 = full0 + kMaxStages * 8;
     const uint32_t acc_full0 = empty0 + kMaxStages * 8, acc_empty0 = acc_full0 + 16;
@@ -605,12 +703,17 @@ __global__ void __launch_bounds__(kThreadsI8, 1) mm8_seq_i8_kernel(const __grid_
             const int nlive = min(a.TT, a.T - t0);                    // tokens of this tile that exist
             RowConst* rc = rowc + (seg & 1) * a.TT;
             // row constants of this tile (its K loop is running meanwhile)
+            bool wide = false;                                        // of any row of this tile
             for (int i = tid; i < a.TT; i += kEpiThreads)
-                if (t0 + i < a.T) rc[i] = a.consts[(size_t)tl.prob * a.T + t0 + i];
+                if (t0 + i < a.T) {
+                    const RowConst r = a.consts[(size_t)tl.prob * a.T + t0 + i];
+                    rc[i] = r;
+                    wide |= r.wide != 0;
+                }
             const bool col = n < p.M;
             const float rxn = col ? __half2float(p.rx[n]) : 0.f, mxn = col ? __half2float(p.mx[n]) : 0.f;
             const float rx128 = rxn * 128.5f;
-            epi_sync();                                               // (and the previous tile's stores have left `tile`)
+            wide = epi_sync_or(wide);                                 // (and the previous tile's stores have left `tile`)
             if (ok) ok = bar_wait(acc_full0 + buf * 8, par);
             if (!ok) *failed = 1;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -627,22 +730,36 @@ __global__ void __launch_bounds__(kThreadsI8, 1) mm8_seq_i8_kernel(const __grid_
 #pragma unroll
                 for (int i = 0; i < 3; ++i) tmem_ld8(d[i], tcol + i * a.TT + c);
             };
+            auto emit = [&](int ti, long long s) {
+                if (whole) put(ti, s);
+                else if (ti < nlive) slot[(size_t)ti * BMC] = s;
+            };
             auto finish = [&](const int (&d)[3][8], int c) {
 #pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    const long long s = (long long)d[2][e] * 65536 + (long long)d[1][e] * 256 + d[0][e];
-                    if (whole) put(c + e, s);
-                    else if (c + e < nlive) slot[(size_t)(c + e) * BMC] = s;
-                }
+                for (int e = 0; e < 8; ++e) emit(c + e, (long long)d[2][e] * 65536 + (long long)d[1][e] * 256 + d[0][e]);
             };
-            if (c_first < nlive) fetch(q[0], c_first);
+            if (__builtin_expect(!wide, 1)) {
+                if (c_first < nlive) fetch(q[0], c_first);
 #pragma unroll
-            for (int k = 0; k < kMaxTT / 32; ++k) {
-                const int c = c_first + 32 * k;
-                if (c >= nlive) break;
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (c + 32 < nlive) fetch(q[(k + 1) & 1], c + 32);
-                finish(q[k & 1], c);
+                for (int k = 0; k < kMaxTT / 32; ++k) {
+                    const int c = c_first + 32 * k;
+                    if (c >= nlive) break;
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (c + 32 < nlive) fetch(q[(k + 1) & 1], c + 32);
+                    finish(q[k & 1], c);
+                }
+            } else {
+#pragma unroll 1
+                for (int c = c_first; c < nlive; c += 32) {
+                    fetch(q[0], c);
+                    tmem_ld8(q[1][0], tcol + 3 * a.TT + c);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        const long long s = (long long)q[0][2][e] * 65536 + (long long)q[0][1][e] * 256 + q[0][0][e];
+                        emit(c + e, rc[c + e].wide ? s * 256 + q[1][0][e] : s);
+                    }
+                }
             }
             // the accumulators are read: the next tile's MMAs may overwrite them
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -743,9 +860,9 @@ __global__ void __launch_bounds__(kThreadsI8, 1) mm8_seq_i8_kernel(const __grid_
                 const CUtensorMap* map = &a.wmap[tl.prob];
                 const int n0 = tl.n0 + (int)crank * BMC, nb = tl.kb1 - tl.kb0;
                 int row = ((tl.prob * a.ntt + tl.tt) * a.nkb + tl.kb0) * xrows;
-                auto load_w = [&](int i, int st) {
+                auto load_w = [&](int i, int st, uint32_t bytes) {
                     if (elect_one()) {
-                        if (crank == 0) bar_expect(full0 + st * 8, PAIR * stage_bytes);
+                        if (crank == 0) bar_expect(full0 + st * 8, PAIR * bytes);
                         if (once) tma_load_2d_hint<PAIR>(smem0 + st * stage_bytes, map, n0, (tl.kb0 + i) * BKI, full_of(st), policy);
                         else tma_load_2d<PAIR>(smem0 + st * stage_bytes, map, n0, (tl.kb0 + i) * BKI, full_of(st));
                     }
@@ -761,26 +878,38 @@ __global__ void __launch_bounds__(kThreadsI8, 1) mm8_seq_i8_kernel(const __grid_
                 int i = 0;
                 if (seg == 0) {                                        // W does not depend on the work before this launch
                     const int ahead = min(S, nb);
-                    for (; i < ahead; ++i) load_w(i, i);
+                    for (; i < ahead; ++i) load_w(i, i, stage_bytes);
                     asm volatile("griddepcontrol.wait;" ::: "memory");
                     asm volatile("fence.proxy.async;" ::: "memory");   // the planes were written by ordinary stores
                     for (int q = 0; q < ahead; ++q) load_x(q);
                     s = ahead == S ? 0 : ahead;
                     ph = ahead == S ? 0u : 1u;
                 }
+                const WideFlags flags = wide_flags(a, tl, lane);
                 for (; i < nb; ++i) {
                     ok = warp_wait(empty0 + s * 8, ph);
                     if (!ok) break;
-                    load_w(i, s);
+                    load_w(i, s, stage_bytes);
                     load_x(s);
                     if (++s == S) { s = 0; ph ^= 1; }
+                }
+                if (__builtin_expect(any_wide(flags), 0)) {            // the K range again, with the fourth plane
+                    const uint32_t bytes = kWTile + (uint32_t)n3 * BKI;
+                    const int lrow = ((tl.prob * a.ntt + tl.tt) * a.nkb + tl.kb0) * a.TT + (int)crank * n3;
+                    for (i = 0; i < nb && ok; ++i) {
+                        ok = warp_wait(empty0 + s * 8, ph);
+                        if (!ok) break;
+                        load_w(i, s, bytes);
+                        if (elect_one()) tma_load_2d<PAIR>(smem0 + s * stage_bytes + kWTile, &a.lmap, 0, lrow + i * a.TT, full_of(s));
+                        if (++s == S) { s = 0; ph ^= 1; }
+                    }
                 }
             }
             if (!ok) *failed = 1;
         }
     } else if (crank == 0) {
         // ================= MMA issuer =================
-        const uint32_t id1 = i8_idesc(BMC * PAIR, a.N1), id2 = i8_idesc(BMC * PAIR, a.N2 ? a.N2 : a.N1);
+        const uint32_t id1 = i8_idesc(BMC * PAIR, a.N1), id2 = i8_idesc(BMC * PAIR, a.N2 ? a.N2 : a.N1), id3 = i8_idesc(BMC * PAIR, a.TT);
         bool ok = true;
         int s = 0;
         uint32_t ph = 0;
@@ -793,6 +922,7 @@ __global__ void __launch_bounds__(kThreadsI8, 1) mm8_seq_i8_kernel(const __grid_
             ok = warp_wait<PAIR == 2>(acc_empty0 + buf * 8, par ^ 1);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t d = tmem + (uint32_t)(buf * a.bufcols);
+            WideFlags flags = {};
             for (int i = 0; i < nb && ok; ++i) {
                 ok = warp_wait(full0 + s * 8, ph);
                 if (!ok) break;
@@ -808,7 +938,27 @@ __global__ void __launch_bounds__(kThreadsI8, 1) mm8_seq_i8_kernel(const __grid_
                     commit_i8<PAIR>(empty0 + s * 8);
                 }
                 __syncwarp();
+                if (i == 0) {                                      // behind the first block's MMAs: asked for before them, the flags cost
+                    if (seg == 0) asm volatile("griddepcontrol.wait;" ::: "memory");     // 1.5 % of a step of 16 rows
+                    flags = wide_flags(a, tl, lane);
+                }
                 if (++s == S) { s = 0; ph ^= 1; }
+            }
+            if (ok && __builtin_expect(any_wide(flags), 0)) {      // the K range again, with the fourth plane
+                for (int i = 0; i < nb && ok; ++i) {
+                    ok = warp_wait(full0 + s * 8, ph);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint64_t ad = ad0 + ((uint32_t)s * stage_bytes >> 4), xd = xd0 + ((uint32_t)s * stage_bytes >> 4);
+                    if (elect_one()) {
+#pragma unroll
+                        for (int j = 0; j < BKI / 32; ++j)
+                            umma_i8<PAIR>(d + 3 * a.TT, ad + (j * 32 * 128 >> 4), xd + (j * 32 >> 4), id3, (i > 0 || j > 0) ? 1u : 0u);
+                        commit_i8<PAIR>(empty0 + s * 8);
+                    }
+                    __syncwarp();
+                    if (++s == S) { s = 0; ph ^= 1; }
+                }
             }
             if (ok && elect_one()) commit_i8<PAIR>(acc_full0 + buf * 8);
             __syncwarp();
@@ -835,7 +985,7 @@ __global__ void __launch_bounds__(kThreadsI8, 1) mm8_seq_i8_kernel(const __grid_
 // ---- host side -------------------------------------------------------------------------------------
 struct Plan {
     int TT, ntt, nkb, pair, N1, N2, stages, smem, units, whole, parts, split, ntiles, bufcols, tmem_cols;
-    size_t tickets, consts, images, slots, bytes;                 // offsets in the workspace, its size
+    size_t tickets, consts, images, low, slots, bytes;                 // offsets in the workspace, its size
 };
 
 // Estimated time of a tile whose K blocks are dealt to `k` CTAs, `ctas` of them at work: a block takes the tensor cores
@@ -844,6 +994,16 @@ double split_cost_us(int nkb, int k, int TT, int ctas) {
     const double block = std::max(std::max(0.28, 0.39 * TT / 128), 0.0025 * ctas);
     return (nkb + k - 1) / k * block + (k > 1 ? 2.5 + 0.02 * TT + 0.1 * k : 0.0);
 }
+
+// A row is wide when three digits would represent it worse than the fp16 path's hi + lo pairs do.  Three digits round each
+// element to a unit (step), so the sum's error relative to the row's norm is sqrt(N / 12) steps over the norm.  The hi + lo
+// path's, measured against fp64 below the fp16 store in rows with a peak above ten times their RMS: 5.2e-7 at N = 768, 9.4e-7
+// to 1.3e-6 at 4096, 2.9e-6 at 16384 (sums in fp32 tensor-core accumulators); of this the fp32 row sums, common to both
+// paths, are 2.5e-7, 4e-7 and 1.2e-6.  The line leaves the total below it; a peak of 5.6 to 12 (N = 768), 12 to 24 (4096) or 31 to
+// 62 times the RMS (16384) crosses it, depending on how it lies to the power of two.  Without a fourth plane a channel 300
+// times the rest cost 1.9e-5 at N = 4096 in columns whose weight there is the middle code, against 9.4e-7 (now 1.3e-6).
+// Returned: the squared norm in steps below which the row is wide.
+float wide_norm(int64_t N) { return float(double(N) / 12 / std::pow(3.6e-7 + 1.1e-10 * double(N), 2)); }
 
 Plan make_plan(int nprob, int64_t T, int64_t N, const int64_t* M, int force) {
     Plan p;
@@ -864,7 +1024,7 @@ Plan make_plan(int nprob, int64_t T, int64_t N, const int64_t* M, int force) {
     const int tail = 512 + p.TT * (2 * int(sizeof(RowConst)) + BMC * 2);
     p.stages = std::min(kMaxStages, (kSmemBudget - 1024 - tail) / stage);
     p.smem = 1024 + p.stages * stage + tail;
-    p.bufcols = n <= 256 ? 256 : 0;
+    p.bufcols = 4 * p.TT <= 256 ? 256 : 0;                         // columns: three planes in two MMAs, then the fourth
     p.tmem_cols = 512;
     p.ntiles = 0;
     for (int i = 0; i < nprob; ++i) p.ntiles += int((M[i] + BMC * pc - 1) / (BMC * pc)) * p.ntt;
@@ -884,7 +1044,8 @@ Plan make_plan(int nprob, int64_t T, int64_t N, const int64_t* M, int force) {
     p.tickets = 1024;
     p.consts = up(p.tickets + size_t(umax) * pc * 4);
     p.images = up(p.consts + size_t(nprob) * T * sizeof(RowConst));
-    p.slots = up(p.images + size_t(nprob) * p.ntt * p.nkb * size_t(n) * BKI);
+    p.low = up(p.images + size_t(nprob) * p.ntt * p.nkb * size_t(n) * BKI);
+    p.slots = up(p.low + size_t(nprob) * p.ntt * p.nkb * size_t(p.TT) * BKI);
     p.bytes = p.slots + (p.split > 1 ? size_t(p.parts) * pc * p.TT * BMC * 8 : 0);
     return p;
 }
@@ -968,6 +1129,7 @@ int rwkv_mm8_seq_i8(int nprob, const SeqI8Problem* probs, int64_t T, int64_t N, 
     if (pro == RWKV_PRO_WKV4 && N % 8 != 0) vec = false;          // rows N apart
     pa.nprob = nprob; pa.vec = vec ? 1 : 0; pa.T = int(T); pa.N = int(N); pa.nkb = p.nkb; pa.TT = p.TT; pa.ntt = p.ntt;
     pa.ntickets = p.split > 1 ? p.parts / p.split * pc : 0;
+    pa.narrow = wide_norm(N); pa.low = ws + p.low;
     pa.images = ws + p.images; pa.consts = reinterpret_cast<RowConst*>(ws + p.consts); pa.tickets = reinterpret_cast<unsigned*>(ws + p.tickets);
     const long long xrows = (long long)nprob * p.ntt * p.nkb * 3 * p.TT;
     if (xrows >= (1ll << 31)) return RWKV_ERR_UNSUPPORTED;
@@ -975,6 +1137,13 @@ int rwkv_mm8_seq_i8(int nprob, const SeqI8Problem* probs, int64_t T, int64_t N, 
         const cuuint64_t dims[2] = {BKI, (cuuint64_t)xrows}, strides[1] = {BKI};
         const cuuint32_t box[2] = {BKI, (cuuint32_t)((i ? p.N2 : p.N1) / pc)}, es[2] = {1, 1};
         if (encode_fn()(&a.xmap[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, pa.images, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return RWKV_ERR_UNSUPPORTED;
+    }
+    {
+        const cuuint64_t dims[2] = {BKI, (cuuint64_t)(xrows / 3)}, strides[1] = {BKI};
+        const cuuint32_t box[2] = {BKI, (cuuint32_t)(p.TT / pc)}, es[2] = {1, 1};
+        if (encode_fn()(&a.lmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, pa.low, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                         CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return RWKV_ERR_UNSUPPORTED;
     }

@@ -330,8 +330,9 @@ int rwkv_mm8_stream_take_error(uint32_t* sync_words, void* stream, int* error_ou
  * accumulation, one rounding to `dtype` at the store (operators.cu:138).
  * Three kernels.  From 2 rows up, fp16 operands whose w rows are 16-byte aligned (pointer, stride; any M, N up
  * to 65536) run on the integer path of the tensor cores (tcgen05 kind::i8, csrc/mm8_seq_i8.cu): the bytes of w
- * as they are, x*ry as 24-bit fixed point per row in three base-256 digits, exact integer sums; results do not
- * depend on the tiling.  From 8 rows up, w that is only 8-byte aligned (pointer, stride, M) runs on the fp16 path
+ * as they are, x*ry as 24-bit fixed point per row in three base-256 digits (32 bits in four for a row whose largest
+ * elements dwarf the rest), exact integer sums; a row's result does not depend on the tiling or on the other rows' values.
+ * From 8 rows up, w that is only 8-byte aligned (pointer, stride, M) runs on the fp16 path
  * (kind::f16, csrc/mm8_seq_tc.cu; x*ry enters as an exact hi + lo pair of fp16 values).  Both need
  * `workspace` = rwkv_mm8_seq_workspace_bytes(B, N, M) bytes, 256-byte aligned, zero when first handed over;
  * everything else (or workspace == NULL) runs on a CUDA-core kernel that accepts any layout.

@@ -81,3 +81,38 @@ def test_range_of_the_fixed_point_scale(ops, magnitude):
     scale = ref.abs().max().item()
     ok = (y.float().cpu() - ref.half().float()).abs() <= ref.abs() * 2 ** -10 + max(scale * 1e-5, 6e-8)
     assert ok[ref.abs() < 6e4].all()
+
+
+# forms: few rows with a K split, pairs of 64 / 96 / 128 tokens with several tiles a CTA, rows read twice (N past one chunk per thread)
+@pytest.mark.parametrize("T,N,M", [(2, 640, 264), (16, 4096, 512), (16, 1024, 40000), (32, 4096, 1000), (40, 4096, 1000), (130, 4096, 640),
+                                   (256, 4096, 9728), (500, 2048, 300), (5, 20480, 136)])
+def test_wide_rows_keep_what_an_outlier_dwarfs(ops, T, N, M):
+    """A row with one huge element: the rest keeps its bits (a fourth digit), which shows in columns whose weight there is zero.
+    W = (q - 128) / 4096 exactly; the other elements are multiples of 2^-8, so that all fp32 row sums are exact."""
+    from chatrwkv_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(T + N + M)
+    q = torch.zeros((N, ops.padded_stride(M)), dtype=torch.uint8, device="cuda")[:, :M]
+    q.copy_(torch.randint(0, 256, (N, M), generator=g, device="cuda"))
+    q[7] = 128
+    c = lambda n, v: torch.full((n,), v, dtype=torch.float16, device="cuda")
+    pack = (q, c(M, -128.5 / 4096), c(M, 2.0 ** -10), c(N, 0.0), c(N, 0.25))
+    x = (torch.randn(T, N, generator=g, device="cuda") * 256).round().div(256).clamp(-4, 4).half()
+    plain, wide = x.clone(), sorted({1, T // 2, T - 1})
+    x[wide, 7] = 60000.0
+
+    def run(a):
+        y = torch.full((T, M), float("nan"), dtype=torch.float16, device="cuda")
+        torch.ops.rwkv.mm8_seq(T, N, M, a, *pack, y)
+        return y
+    y = run(x)
+    ref = (x.double() @ (q.double() - 128)) / 4096
+    # the store's rounding, and one fp32 rounding of mx * SX = 1882 (half a step: 2^-14); three digits alone miss by 1e-2
+    assert ((y.double() - ref).abs() <= ref.abs() * 2 ** -11 * 1.001 + 2 ** -13)[wide].all()
+    others = [t for t in range(T) if t not in wide]
+    assert torch.equal(y[others], run(plain)[others])           # a wide row changes no other row
+    _lib.lib().rwkv_mm8_seq_set_path(8)
+    try:
+        assert torch.equal(y, run(x))                           # one CTA per tile: the same bits
+    finally:
+        _lib.lib().rwkv_mm8_seq_set_path(0)
+    assert _error_word(ops) == 0
