@@ -253,8 +253,9 @@ class RWKV:
                 args.n_head = w["blocks.0.att.time_first"].shape[0]
             # the fused one-token path and the batched path are built for int8 matrices throughout; a model with plain
             # fp16 layers runs every call through the sequence path (library GEMMs for those layers)
-            self._all_i8 = all(w[k].dtype == torch.uint8 for k in w
-                               if torch.is_tensor(w[k]) and any(sk in k for sk in _MATRIX_KEYS) and k.endswith(".weight"))
+            i8 = [w[k].dtype == torch.uint8 for k in w
+                  if torch.is_tensor(w[k]) and any(sk in k for sk in _MATRIX_KEYS) and k.endswith(".weight")]
+            self._all_i8, self._any_i8 = all(i8), any(i8)
             self._full_m = {}
             if self._world > 1:
                 if self.version != 4:
@@ -1256,10 +1257,22 @@ class RWKV:
         which hands it out again only when the copy is over (calls of several threads never share one)."""
         return torch.tensor(tokens, dtype=torch.int64, pin_memory=True).to(self.device, non_blocking=True)
 
-    # The group norm of RWKV-5/6 divides by nearly nothing at the first positions of an empty state: there two correct
-    # summation orders of the same matmul end up percents apart, and the difference fades as 1 / T (state entries: 0.4 of
-    # their RMS after 100 tokens, 0.05 after 600).  Shorter prompts from an empty state keep the fp16 path's sums.
+    # The group norm of RWKV-5/6 divides by nearly nothing at the first positions of an empty state: there two correct sums of
+    # the same matmul end up percents apart after 32 layers, and the difference fades as 1 / T (state entries: 0.4 of their RMS
+    # after 100 tokens, 0.05 after 600).  Neither sum is the better one (6 layers of 4096, against fp32 activations: 12 tokens
+    # 2.42e-2 on the fp16 path and 2.39e-2 on the integer path, 100 tokens 3.65e-3 and 3.64e-3, 600 tokens 1.52e-3 and 1.22e-3).
+    # So that the answers to such prompts do not change with the kernel, those that start from the initial state and are
+    # shorter than this keep the sums of the fp16 path; longer ones, and chunks on a state, take the faster kernel.
     EARLY_PROMPT = 512
+
+    def _is_initial(self, state):
+        """Whether an RWKV-5/6 state is what `None` stands for, read from the first layer's matrix state (any token changes it).
+        One small reduction, and the host waits for it; under stream capture nothing can be read and the answer is no."""
+        if torch.cuda.is_current_stream_capturing():
+            return False
+        if self.args.time_state:
+            return torch.equal(state[1], self._zero_state()[1])
+        return not state[1].any().item()
 
     def _forward_seq(self, tokens, state, full_output, fresh=False):
         # (Replaying a prompt length that comes back as a CUDA graph was tried: with the copies of the state in and out
@@ -1267,7 +1280,7 @@ class RWKV:
         w, a = self.w, self.args
         state = list(state)
         idx = self._stage_tokens(tokens)
-        early = fresh and self.version != 4 and len(tokens) < self.EARLY_PROMPT
+        early = self.version != 4 and len(tokens) < self.EARLY_PROMPT and (fresh or (self._any_i8 and self._is_initial(state)))
         x = w["emb.weight"].index_select(0, idx)
         for i in range(a.n_layer):
             if self.version == 4:
