@@ -16,8 +16,8 @@ TOL = 2e-2
 @pytest.mark.parametrize("B", [3, 9])
 @pytest.mark.parametrize("name", ["v4", "v5", "v6"])
 def test_forward_batch_matches_per_sequence_decode(name, B):
-    """B = 3 runs the CUDA-core mm8_seq kernel, B = 9 the tensor-core one.  Sequences start from different prompts
-    (stack_states of B prefills), decode 6 tokens each."""
+    """Both batch sizes run the integer tensor-core kernel with the prologues in its operand pass.  Sequences start from
+    different prompts (stack_states of B prefills), decode 6 tokens each."""
     from chatrwkv_b200.model import RWKV
     ck = synth.make_checkpoint(**TOY[name])
     V = TOY[name]["vocab"]

@@ -273,11 +273,32 @@ def test_op_schemas(ops):
             assert hasattr(ns, f)
 
 
+def _mm8_seq_on(ops, kernel, x, pack, y):
+    """mm8_seq on a named tensor-core kernel: "i8" (16-byte aligned rows of w: the default), "f16" (the hi + lo form asked for
+    by SEQ_F16_SUMS) or "f16-8byte" (the same, which rows that start on 8 bytes only get by themselves)."""
+    from chatrwkv_b200 import _lib
+    if kernel == "f16-8byte":
+        q = pack[0]
+        M = q.shape[1]
+        wide = torch.zeros((q.shape[0], (M + 15) // 16 * 16 + 8), dtype=torch.uint8, device=q.device)[:, :M]
+        wide.copy_(q)
+        pack = (wide,) + tuple(pack[1:])
+    if kernel == "f16":
+        return ops.mm8_seq_epi(x, *pack, y, _lib.EPI_STORE | _lib.SEQ_F16_SUMS)
+    torch.ops.rwkv.mm8_seq(x.shape[0], x.shape[1], y.shape[1], x, *pack, y)
+    return y
+
+
+KERNELS = ["i8", "f16", "f16-8byte"]
+
+
+@pytest.mark.parametrize("kernel", KERNELS)
 @pytest.mark.parametrize("T,N,M", [(128, 256, 128), (64, 64, 128), (200, 768, 3072), (1024, 4096, 512), (257, 1000, 264),
                                    (130, 100, 304), (13, 4104, 512)])
-def test_mm8_seq_tensor_core_path(ops, T, N, M):
-    """Rows >= 8 with an 8-byte-aligned matrix run on tcgen05; same oracle, same tolerance.
-    Includes ragged T (not a multiple of 128 or 8), N (not a multiple of 64 or 8) and M (not of 128)."""
+def test_mm8_seq_tensor_core_path(ops, T, N, M, kernel):
+    """Rows >= 8 with an 8-byte-aligned matrix run on tcgen05 (the integer kernel where rows start on 16 bytes, else the fp16
+    one); same oracle, same tolerance.  Includes ragged T (not a multiple of 128 or 8), N (not a multiple of 64 or 8) and M
+    (not of 128), and launches of the fp16 kernel with a K split (13 x 4104 x 512, 1024 x 4096 x 512)."""
     import ctypes
     from chatrwkv_b200 import _lib
     from tests.util import packed_case
@@ -286,7 +307,7 @@ def test_mm8_seq_tensor_core_path(ops, T, N, M):
     x = torch.randn(T, N, generator=g).half()
     ref = orc.mm8_kernel(x, *cpu)
     y = torch.empty((T, M), dtype=torch.float16, device="cuda")
-    torch.ops.rwkv.mm8_seq(T, N, M, x.cuda(), *dev, y)
+    _mm8_seq_on(ops, kernel, x.cuda(), dev, y)
     torch.cuda.synchronize()
     ws = ops.workspace(torch.device("cuda", torch.cuda.current_device()), 1024, "mm8_seq")
     e = ctypes.c_int(0)
@@ -305,12 +326,13 @@ def test_mm8_seq_tensor_core_path(ops, T, N, M):
     assert ((y.float() - y2.float()).abs() <= y2.float().abs() * 2 ** -9 + 2e-4).all()
 
 
+@pytest.mark.parametrize("kernel", KERNELS)
 @pytest.mark.parametrize("T,N,M", [(256, 320, 9728), (200, 200, 19464), (512, 128, 5000 * 8), (1024, 4096, 4096)])
-def test_mm8_seq_cta_pair_form(ops, T, N, M):
-    """Launches with an even number of 128-row tiles and no K split (more output tiles than half of the SMs) run as
-    clusters of two CTAs that share one 256-row UMMA (tcgen05 cta_group::2), each converting half of the B tile.
-    Same sums in the same order: bit-identical to the one-CTA form (set_path bit 3), and both match the oracle.
-    Includes a ragged last row tile and ragged N and M."""
+def test_mm8_seq_cta_pair_form(ops, T, N, M, kernel):
+    """The fp16 kernel: launches with an even number of 128-row tiles and no K split (more output tiles than half of the SMs)
+    run as clusters of two CTAs that share one 256-row UMMA (tcgen05 cta_group::2), each converting half of the B tile.  The
+    integer kernel: launches of more than 32 rows.  Same sums (in the same order, or exact): bit-identical to the one-CTA form
+    (set_path bit 3), and both match the oracle.  Includes a ragged last row tile and ragged N and M."""
     import ctypes
     from chatrwkv_b200 import _lib
     from tests.util import packed_case
@@ -319,11 +341,11 @@ def test_mm8_seq_cta_pair_form(ops, T, N, M):
     x = torch.randn(T, N, generator=g).half()
     xd = x.cuda()
     y = torch.empty((T, M), dtype=torch.float16, device="cuda")
-    torch.ops.rwkv.mm8_seq(T, N, M, xd, *dev, y)
+    _mm8_seq_on(ops, kernel, xd, dev, y)
     _lib.lib().rwkv_mm8_seq_set_path(8)
     try:
         y1 = torch.empty_like(y)
-        torch.ops.rwkv.mm8_seq(T, N, M, xd, *dev, y1)
+        _mm8_seq_on(ops, kernel, xd, dev, y1)
     finally:
         _lib.lib().rwkv_mm8_seq_set_path(0)
     torch.cuda.synchronize()
@@ -337,9 +359,10 @@ def test_mm8_seq_cta_pair_form(ops, T, N, M):
         assert (err <= ref.abs() * 2 ** -10 + 1e-4).all(), err.max().item()
 
 
-def test_mm8_seq_ignores_stale_scratch_rows(ops):
-    """The operand images keep whatever the scratch held in the rows past T of the last 128-row tile
-    (here: NaN patterns); no stored output may depend on them."""
+@pytest.mark.parametrize("kernel", KERNELS)
+def test_mm8_seq_ignores_stale_scratch_rows(ops, kernel):
+    """The operand images keep whatever the scratch held in the rows past T of the last row tile (here: NaN patterns, which
+    are -1 as the integer kernel's digits, then another fill); no stored output may depend on them."""
     from tests.util import packed_case
     T, N, M = 130, 512, 256
     cpu, dev = packed_case(N, M, seed=5)
@@ -347,15 +370,19 @@ def test_mm8_seq_ignores_stale_scratch_rows(ops):
     x = torch.randn(T, N, generator=g).half()
     ref = orc.mm8_kernel(x, *cpu)
     y = torch.empty((T, M), dtype=torch.float16, device="cuda")
-    torch.ops.rwkv.mm8_seq(T, N, M, x.cuda(), *dev, y)              # sizes the scratch
+    _mm8_seq_on(ops, kernel, x.cuda(), dev, y)                      # sizes the scratch
     torch.cuda.synchronize()
     ws = ops.workspace(torch.device("cuda", torch.cuda.current_device()), 1024, "mm8_seq")
     ws[256:8 << 20].fill_(0xFF)                                       # fp16 / fp32 NaN everywhere but the error word
     y.zero_()
-    torch.ops.rwkv.mm8_seq(T, N, M, x.cuda(), *dev, y)
+    _mm8_seq_on(ops, kernel, x.cuda(), dev, y)
     torch.cuda.synchronize()
     assert torch.isfinite(y).all()
     assert ((y.float().cpu() - ref).abs() <= ref.abs() * 2 ** -10 + 1e-4).all()
+    ws[256:8 << 20].fill_(0x3B)
+    y1 = torch.zeros_like(y)
+    _mm8_seq_on(ops, kernel, x.cuda(), dev, y1)
+    assert torch.equal(y, y1)
     ws[256:8 << 20].zero_()
 
 
