@@ -114,7 +114,7 @@ extern "C" void rwkv_mm8_seq_set_path(int path) {
     g_seq_single = (path & 4) != 0;
     rwkv_mm8_seq_tc_set_single(g_seq_single);
     rwkv_mm8_seq_tc_set_no_pair((path & 8) != 0);
-    rwkv_mm8_seq_i8_set_form((path & 8) != 0 ? 1 : 0);
+    rwkv_mm8_seq_i8_set_single_cta((path & 8) != 0);
 }
 constexpr int kI8MinRows = 2;   // one row is mm8_one's work; from two on the integer tensor-core kernel (4096 x 4096: 11 us)
 constexpr int kTcMinRows = 8;   // rows that TMA cannot fetch: below this the CUDA-core kernel, from here on the 128-row fp16 tile

@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(MAXT, MINB) mm8_seq_i8_prep(const __grid_const
         const HV<E> g = load_hv<E>(static_cast<const __half*>(q.gate) + (long long)t * q.gate_stride, k0, N, vec);
         load_f<E>(static_cast<const float*>(q.ln_w), k0, N, vec, gw);
         load_f<E>(static_cast<const float*>(q.ln_b), k0, N, vec, gb);
-        const int per = q.head / E;                       // threads of a head: 1, 2, 4 or 8 neighbouring lanes
+        const int per = q.head / E;                       // threads of a head: 1 to 32 neighbouring lanes (128 channels, E = 4)
         float s = 0.f, v = 0.f;
 #pragma unroll
         for (int e = 0; e < E; ++e) s += y[e];
@@ -1005,7 +1005,7 @@ double split_cost_us(int nkb, int k, int TT, int ctas) {
 // Returned: the squared norm in steps below which the row is wide.
 float wide_norm(int64_t N) { return float(double(N) / 12 / std::pow(3.6e-7 + 1.1e-10 * double(N), 2)); }
 
-Plan make_plan(int nprob, int64_t T, int64_t N, const int64_t* M, int force) {
+Plan make_plan(int nprob, int64_t T, int64_t N, const int64_t* M, bool single) {
     Plan p;
     const int sms = rwkv_sm_count();
     p.nkb = int((N + BKI - 1) / BKI);
@@ -1013,7 +1013,7 @@ Plan make_plan(int nprob, int64_t T, int64_t N, const int64_t* M, int force) {
     const int per = int((T + p.ntt - 1) / p.ntt);
     // Pairs halve the token planes each CTA fetches and reads; up to 32 rows these are small and single CTAs spread a matrix
     // over twice as many units (4096 x 4096: 16 rows 13.9 against 15.0 us, 64 rows equal, 1024 rows 64 against 56 us).
-    p.pair = force == 1 ? 0 : force == 2 ? 1 : (per > 32 ? 1 : 0);
+    p.pair = !single && per > 32 ? 1 : 0;
     const int unit = p.pair ? 32 : 16;
     p.TT = (per + unit - 1) / unit * unit;
     const int n = 3 * p.TT;
@@ -1065,15 +1065,15 @@ EncodeFn encode_fn() {
     return fn;
 }
 
-int g_i8_form = 0;                       // 0 automatic, 1 one CTA per tile, 2 pairs (set through rwkv_mm8_seq_set_path)
+bool g_i8_single = false;                // one CTA per tile always (set through rwkv_mm8_seq_set_path)
 
 }  // namespace
 
-void rwkv_mm8_seq_i8_set_form(int form) { g_i8_form = form; }
+void rwkv_mm8_seq_i8_set_single_cta(bool single) { g_i8_single = single; }
 
 size_t rwkv_mm8_seq_i8_workspace_bytes(int nprob, int64_t T, int64_t N, const int64_t* M) {
     if (nprob < 1 || nprob > kSeqI8MaxProblems || T < 1 || N < 1 || N > 65536) return 0;
-    return std::max(make_plan(nprob, T, N, M, 1).bytes, make_plan(nprob, T, N, M, 2).bytes);
+    return std::max(make_plan(nprob, T, N, M, false).bytes, make_plan(nprob, T, N, M, true).bytes);
 }
 
 int rwkv_mm8_seq_i8(int nprob, const SeqI8Problem* probs, int64_t T, int64_t N, void* workspace, size_t workspace_bytes, void* stream) {
@@ -1088,7 +1088,7 @@ int rwkv_mm8_seq_i8(int nprob, const SeqI8Problem* probs, int64_t T, int64_t N, 
     if (encode_fn() == nullptr) return RWKV_ERR_UNSUPPORTED;
     static int use_pair = -1;            // RWKV_B200_SEQ_PAIR=0: never the CTA-pair form (same results)
     if (use_pair < 0) { const char* e = getenv("RWKV_B200_SEQ_PAIR"); use_pair = (e != nullptr && e[0] == '0') ? 0 : 1; }
-    const Plan p = make_plan(nprob, T, N, M, use_pair ? g_i8_form : 1);
+    const Plan p = make_plan(nprob, T, N, M, !use_pair || g_i8_single);
     if (workspace == nullptr || workspace_bytes < p.bytes) return RWKV_ERR_WORKSPACE;
     RWKV_CHECK_ALIGN(workspace, 256);
     uint8_t* ws = static_cast<uint8_t*>(workspace);

@@ -15,4 +15,4 @@ struct SeqI8Problem {
 size_t rwkv_mm8_seq_i8_workspace_bytes(int nprob, int64_t T, int64_t N, const int64_t* M);
 // fp16 operands; RWKV_ERR_UNSUPPORTED when a layout is not one TMA can fetch (the caller then takes another kernel).
 int rwkv_mm8_seq_i8(int nprob, const SeqI8Problem* probs, int64_t T, int64_t N, void* workspace, size_t workspace_bytes, void* stream);
-void rwkv_mm8_seq_i8_set_form(int form);       // 0 automatic, 1 single CTAs, 2 CTA pairs (results are identical)
+void rwkv_mm8_seq_i8_set_single_cta(bool single);       // never CTA pairs (same results)

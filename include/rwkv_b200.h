@@ -331,7 +331,8 @@ int rwkv_mm8_stream_take_error(uint32_t* sync_words, void* stream, int* error_ou
  * Three kernels.  From 2 rows up, fp16 operands whose w rows are 16-byte aligned (pointer, stride; any M, N up
  * to 65536) run on the integer path of the tensor cores (tcgen05 kind::i8, csrc/mm8_seq_i8.cu): the bytes of w
  * as they are, x*ry as 24-bit fixed point per row in three base-256 digits (32 bits in four for a row whose largest
- * elements dwarf the rest), exact integer sums; a row's result does not depend on the tiling or on the other rows' values.
+ * elements dwarf the rest), exact integer sums, which depend neither on the tiling nor on the other rows (the fp32 sums of x,
+ * x*ry and x*my run in an order that depends on the launch's rows).
  * From 8 rows up, w that is only 8-byte aligned (pointer, stride, M) runs on the fp16 path
  * (kind::f16, csrc/mm8_seq_tc.cu; x*ry enters as an exact hi + lo pair of fp16 values).  Both need
  * `workspace` = rwkv_mm8_seq_workspace_bytes(B, N, M) bytes, 256-byte aligned, zero when first handed over;
@@ -370,7 +371,8 @@ int rwkv_mm8_seq(int64_t B, int64_t N, int64_t M, const void* x, int64_t x_strid
  *                     LayerNorm, then per problem the token-shift `mix` [N] (rwkv_ln_mix: mode 0 RWKV-4/5, mode 1 RWKV-6;
  *                     mode 2: the LayerNorm alone).  sx_stride == 0: the rows are consecutive tokens, sx [N] the state before the
  *                     first; else row t is a sequence of its own with its state at sx + t * sx_stride.  xx_out (may be
- *                     NULL): the LayerNorm output of every row; new_state (may be NULL): that of the last row.
+ *                     NULL): the LayerNorm output of every row; new_state (may be NULL): that of the last row (neither may
+ *                     alias x or sx).
  *   RWKV_PRO_WKV4     one problem: x = r [B, N], one step of the RWKV-4 recurrence per row on the states aa, bb, pp [B, N]
  *                     (updated in place), k, v [B, N] fp16; the matmul's row is r * wkv (rwkv_wkv4_seq with T = 1).
  *   RWKV_PRO_GN_GATE  one problem: x [B, N] in fp32, group norm over each `head` channels with eps and ln_w, ln_b in
