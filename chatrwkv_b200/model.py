@@ -1174,7 +1174,8 @@ class RWKV:
         batch state).  The B sequences are the rows of the tensor-core mm8_seq kernel, so the packed weights are
         streamed once per step for all of them; every sequence follows the arithmetic of the prefill path with T = 1.
         The RWKV-4 WKV states (aa, bb, pp) are updated in place, everything else is returned in new tensors (with
-        graphs, in the tensors that _forward_batch_graph names)."""
+        graphs, in the tensors that _forward_batch_graph names).  All steps run the integer matmul kernel, the first ones of
+        RWKV-5/6 sequences among them (EARLY_PROMPT is a rule for prompts)."""
         if self._world > 1:
             raise NotImplementedError("forward_batch: single-GPU models only")
         with torch.no_grad(), torch.cuda.device(self.device):
@@ -1186,10 +1187,11 @@ class RWKV:
             return self._forward_batch_eager(idx, state)
 
     def _forward_batch_graph(self, idx, state):
-        """forward_batch as one CUDA-graph replay per batch size.  The graph reads the state from fixed input tensors
-        and leaves the new state in fixed output tensors (its first node copies outputs back to inputs), so the list
-        it returns is overwritten by the next call with the same batch size: pass copy.deepcopy(state) around to keep
-        a snapshot, as with the one-token forward."""
+        """forward_batch as one CUDA-graph replay per batch size.  The graph reads the state from fixed input tensors, which
+        every call fills before the replay (from the last call's outputs, or from the caller's state).  The recurrences' states
+        are updated in those tensors, the shift states land in fixed output tensors; the list returned holds both, so it is
+        overwritten by the next call with the same batch size: pass copy.deepcopy(state) around to keep a snapshot, as with
+        the one-token forward."""
         B = idx.numel()
         g = self._batch_graphs.get(B)
         if g is None:
